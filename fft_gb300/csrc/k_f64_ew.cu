@@ -40,7 +40,7 @@ __global__ void real_pass_kernel64(const RealPassParams p) {
   }
   if (q >= p.nlines || k >= half) return;
   const long long L = p.L;
-  const double2* rtw = reinterpret_cast<const double2*>(p.rtw);
+  const int4* rtw = reinterpret_cast<const int4*>(p.rtw);
   const long long bi = line_off(p.in, q), bo = line_off(p.out, q);
   const long long ik = bi + k * p.in.es, iL = bi + (L - k) * p.in.es;
   const long long ok = bo + k * p.out.es, oL = bo + (L - k) * p.out.es;
@@ -56,8 +56,8 @@ __global__ void real_pass_kernel64(const RealPassParams p) {
       oim[oL] = 0.0;
       return;
     }
-    const double2 xk = post_one64(s0, s1, rtw[k]);
-    const double2 xl = post_one64(s1, s0, rtw[L - k]);
+    const double2 xk = post_one64(s0, s1, ldz(rtw + k));
+    const double2 xl = post_one64(s1, s0, ldz(rtw + L - k));
     ore[ok] = xk.x;
     oim[ok] = xk.y;
     if (L - k != k) {
@@ -70,8 +70,8 @@ __global__ void real_pass_kernel64(const RealPassParams p) {
       oim[ok] = s0.x - s1.x;
       return;
     }
-    const double2 zk = pre_one64(s0, s1, rtw[k]);
-    const double2 zl = pre_one64(s1, s0, rtw[L - k]);
+    const double2 zk = pre_one64(s0, s1, ldz(rtw + k));
+    const double2 zl = pre_one64(s1, s0, ldz(rtw + L - k));
     ore[ok] = zk.x;
     oim[ok] = zk.y;
     if (L - k != k) {

@@ -1,7 +1,7 @@
 // Registry entries of the FP64 line kernels (line_fft64.cuh).
 #pragma once
 #include "kernels.h"
-#include "line_fft64.cuh"
+#include "line_fx64.cuh"
 
 namespace agb {
 
@@ -9,7 +9,10 @@ template <int LOGL, bool COLS, int KIND, bool TSTORE>
 LineKernel make_line_kernel64() {
   constexpr int C = lines_per_cta64<LOGL, COLS>();
   LineKernel k{};
-  k.fn = &line_fft64<LOGL, C, COLS, KIND, TSTORE>;
+  // lines of up to 4 points stay on the FP64 pipe: 2 to 4 additions per
+  // point there against the conversions to and from fixed point
+  if constexpr (LOGL >= 3) k.fn = &line_fx64<LOGL, C, COLS, KIND, TSTORE>;
+  else k.fn = &line_fft64<LOGL, C, COLS, KIND, TSTORE>;
   k.grouped = nullptr;
   k.logl = LOGL;
   k.cols = COLS;

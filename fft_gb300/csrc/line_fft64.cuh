@@ -7,14 +7,15 @@
 // sized for FP64: each thread owns E = 8 complex doubles of one line in the
 // canonical layout v[e] = x[t + T*e] (T = L/8), and the stages are radix-8,
 // with one radix-2 or radix-4 stage first when log2 L is not a multiple of 3.
-// On GB300 FP64 arithmetic, not HBM, bounds these transforms (two FP64 FMA
-// lanes per SM per clock, 1/64 of the FP32 rate), and radix-8 stages cost
-// about as many FP64 instructions per point and log2 L as radix-16 ones
-// (3.5 vs 3.4) with half the registers.
+// On GB300 FP64 arithmetic, not HBM, bounds these transforms on the FP64 pipe
+// (two FMA lanes per SM per clock, 1/64 of the FP32 rate), so lines of 8
+// points and more run in block fixed point (line_fx64.cuh, same schedule,
+// layouts and tables); the FP64 body here serves shorter lines and the values
+// that form does not take.
 //
-// Twiddles are FP64 tables computed on the host (no rounding step).  They
-// travel in the LineParams / RealPassParams table fields (tw, tw_full, rtw),
-// which point to double2 arrays for these kernels; the four-step twiddle
+// Twiddles are computed in FP64 on the host and kept in 62-bit fixed point.
+// They travel in the LineParams / RealPassParams table fields (tw, tw_full,
+// rtw), which point to int4 arrays for these kernels; the four-step twiddle
 // always comes from the full matrix table tw_full[t2 * L + k].
 #pragma once
 
@@ -46,12 +47,15 @@ struct Sched64 {
 
 // Lines per CTA: rows as the FP32 kernels (256 threads, or one line of up to
 // 1024 threads); cols 2048 points per tile up to 256-point lines (256
-// threads), 8 lines at 512 and 1024 points (64-byte row segments), 4 at 2048
-// (32-byte segments, 128 KB of shared memory).
+// threads), 8 lines at 512 points (64-byte row segments), 4 at 1024 and 2048
+// (32-byte segments; 64 and 128 KB of shared memory: two 1024-point tiles
+// per SM, one's work under the other's barriers, 16 x 2^20 c2c 0.584 vs
+// 0.731 ms with 8 lines; 2 lines at 2048 points 2048^2 c2c 4% faster, 4096^2
+// c2r 11% slower).
 template <int LOGL, bool COLS>
 constexpr int lines_per_cta64() {
   constexpr int L = 1 << LOGL, T = Sched64<LOGL>::T;
-  if constexpr (COLS) return L <= 8 ? 256 : (L <= 256 ? 2048 / L : (L <= 1024 ? 8 : 4));
+  if constexpr (COLS) return L <= 8 ? 256 : (L <= 256 ? 2048 / L : (L <= 512 ? 8 : 4));
   else return T >= 256 ? 1 : 256 / T;
 }
 
@@ -69,7 +73,13 @@ __device__ __forceinline__ double2 zsub(double2 a, double2 b) { return make_doub
 __device__ __forceinline__ double2 zconj(double2 a) { return make_double2(a.x, -a.y); }
 __device__ __forceinline__ double2 zmul_negi(double2 a) { return make_double2(a.y, -a.x); }   // -i*a
 __device__ __forceinline__ double2 zswap(double2 a) { return make_double2(a.y, a.x); }
-__device__ __forceinline__ double2 ldz(const double2* p) { return __ldg(p); }
+// A root of unity from its fixed-point table entry (root_d in plan.cu): the
+// value is ((re high) * 2^32 + re low) / 2^62, likewise im.
+__device__ __forceinline__ double2 ldz(const int4* p) {
+  const int4 w = __ldg(p);
+  return make_double2((double)((long long)w.x * (1LL << 32) + w.y) * 0x1p-62,
+                      (double)((long long)w.z * (1LL << 32) + w.w) * 0x1p-62);
+}
 
 #define AFFT_R2D 0.70710678118654752440   // sqrt(1/2)
 
@@ -142,7 +152,7 @@ struct Smem64 {
 // slots u + B*r, applies W_{NS R}^{r (b mod NS)}, DFT-R, and scatters to
 // shared memory (non-last) or keeps the canonical layout (last).
 template <int R, int NS, int E, int T, bool LAST, class SM>
-__device__ __forceinline__ void stage64(double2 (&v)[E], int t, int c, const double2* tw, const SM& sm) {
+__device__ __forceinline__ void stage64(double2 (&v)[E], int t, int c, const int4* tw, const SM& sm) {
   constexpr int B = E / R;
 #pragma unroll
   for (int u = 0; u < B; u++) {
@@ -168,7 +178,7 @@ __device__ __forceinline__ void stage64(double2 (&v)[E], int t, int c, const dou
 }
 
 template <int LOGL, bool WARP_ONLY, int S, class SM>
-__device__ __forceinline__ void run_stages64(double2 (&v)[Sched64<LOGL>::E], int t, int c, const double2* tw,
+__device__ __forceinline__ void run_stages64(double2 (&v)[Sched64<LOGL>::E], int t, int c, const int4* tw,
                                              const SM& sm) {
   using Sc = Sched64<LOGL>;
   if constexpr (S < Sc::NSTAGES) {
@@ -205,8 +215,8 @@ __device__ __forceinline__ void line_fft64_body(const LineParams& p, long long c
   constexpr bool WARP_ONLY = (!COLS && T <= 32) || (T * C <= 32);
   extern __shared__ __align__(1024) double2 smem64[];
   Smem64<L, C, COLS> sm{smem64};
-  const double2* tw = reinterpret_cast<const double2*>(p.tw);
-  const double2* rtw = reinterpret_cast<const double2*>(p.rtw);
+  const int4* tw = reinterpret_cast<const int4*>(p.tw);
+  const int4* rtw = reinterpret_cast<const int4*>(p.rtw);
 
   const int tid = threadIdx.x;
   const int c = COLS ? (tid % C) : (tid / T);
@@ -265,7 +275,7 @@ __device__ __forceinline__ void line_fft64_body(const LineParams& p, long long c
     const long long q2 = cta * C + c2;
     if (q2 < p.nlines) {
       const long long base = line_off(p.out, q2);
-      const double2* twf = reinterpret_cast<const double2*>(p.tw_full);
+      const int4* twf = reinterpret_cast<const int4*>(p.tw_full);
       const int r2 = (int)((q2 >> p.tw_qshift) & p.tw_qmask);
 #pragma unroll
       for (int e = 0; e < E; e++) {
@@ -281,7 +291,7 @@ __device__ __forceinline__ void line_fft64_body(const LineParams& p, long long c
   } else if constexpr (KIND == LK_C2C) {
     if constexpr (COLS) {
       if (p.tw_n) {
-        const double2* twf = reinterpret_cast<const double2*>(p.tw_full);
+        const int4* twf = reinterpret_cast<const int4*>(p.tw_full);
         const int r2 = (int)((q >> p.tw_qshift) & p.tw_qmask);
 #pragma unroll
         for (int e = 0; e < E; e++) v[e] = zmul(v[e], ldz(twf + (long long)r2 * L + t + T * e));
@@ -348,7 +358,7 @@ __global__ void __launch_bounds__(Sched64<LOGL>::T * C) line_fft64(const LinePar
 }
 
 // FP64 forms of the standalone real pass, the line copy and the size-1 real
-// transform (the FP32 ones are in real_pass.cu); their table is double2.
+// transform (the FP32 ones are in real_pass.cu); their table is int4 (62-bit fixed point).
 __global__ void real_pass_kernel64(const RealPassParams p);
 __global__ void copy_lines_kernel64(const CopyParams p);
 __global__ void real1_kernel64(const RealPassParams p);

@@ -1,0 +1,472 @@
+// FP64 lines computed in 64-bit block fixed point on the integer pipes.
+//
+// GB300 has two FP64 lanes per SM and clock against 64 lanes each of 64-bit
+// integer adds and of 32x32+64-bit multiply-adds (measured: add.s64 59,
+// mad.wide.s32 60, DADD 1.7, cvt to and from f64 2.0 results per SM and
+// clock).  An FP64 transform that runs on the FP64 pipe is bound by it at
+// about a tenth of what HBM allows.  Here a line's doubles become 64-bit
+// integers that share one exponent, the stages run on those, and the results
+// are rounded to double once at the end.
+//
+// Precision.  A line's values are held with the largest one's top bit at
+// bit 57 to 60, so the unit is at most 2^-57 of the line's largest value,
+// against 2^-53 relative roundoff per FP64 operation.  Between two stages the
+// line is shifted (by the OR of all magnitudes, so no headroom is spent that
+// the data do not need) to keep it that way.  Products by a twiddle use its
+// 62-bit fixed-point value; the low x low partial product, at most a quarter
+// unit, is dropped.  The error is therefore relative to the line's norm, as
+// that of the FP64 butterflies is, and smaller: against extended-precision
+// FFTs of normal data 0.86e-16 at 4096 points (FP64: 2.4e-16), 1.2e-16 at
+// 2^17 (2.8e-16); with one value 1e5 times the others 1.4 to 2.0e-16 (2.2 to
+// 2.8e-16).
+//
+// Range.  Lines with a non-finite value, one above 2^977, or nonzero data
+// below 2^-823 are left to the FP64 body of the same kernel (the whole CTA
+// takes it), so infinities, NaNs, overflow and subnormals behave as there.
+//
+// Bounds, in bits (component magnitudes; |z| is the complex magnitude): first
+// stage's output |z| < 2^62.5, every intermediate < 2^63; before a twiddle
+// product the line is shifted so that its top bit is bit 59 (components
+// < 2^60, |z| < 2^60.5); the product is scaled by 1/4: |z| < 2^58.5, and
+// < 2^61.5 after the next radix-8 stage.
+#pragma once
+
+#include "line_fft64.cuh"
+
+namespace agb {
+
+typedef long long fx;
+
+struct fxc {
+  fx x, y;
+};
+
+// bit of the largest input component's leading one: as high as the first
+// stage's growth allows (output |z| < 2^62.5; a lone radix-8 stage, whose
+// output the real post-pass adds in pairs, one lower)
+template <int LOGL>
+constexpr int fx_top() {
+  using Sc = Sched64<LOGL>;
+  return Sc::FIRST == 2 ? 60 : Sc::FIRST == 4 ? 59 : Sc::NSTAGES > 1 ? 58 : 57;
+}
+constexpr int FX_TOP_TW = 59;     // the same where a twiddle product follows
+constexpr int FX_EXP_MIN = 200;   // biased exponents the fixed-point form takes: below, subnormal results are
+constexpr int FX_EXP_MAX = 2000;  // possible; above, overflow (14 bits of growth) and non-finite values
+
+__device__ __forceinline__ int fx_hi(fx a) { return (int)(a >> 32); }
+__device__ __forceinline__ int fx_lo(fx a) { return (int)a; }
+// a = fx_s1(a) * 2^32 + (signed) fx_lo(a)
+__device__ __forceinline__ int fx_s1(fx a) { return fx_hi(a) + (int)((unsigned)fx_lo(a) >> 31); }
+__device__ __forceinline__ fx mw(int a, int b) { return (fx)a * (fx)b; }
+
+// a / 2^n to nearest, ties away from zero: a mean of half a tie would add up
+// over a line to an error in bin 0
+__device__ __forceinline__ fx fx_sar(fx a, int n) { return (a + (1LL << (n - 1)) + (a >> 63)) >> n; }
+
+__device__ __forceinline__ fxc cadd(fxc a, fxc b) { return {a.x + b.x, a.y + b.y}; }
+__device__ __forceinline__ fxc csub(fxc a, fxc b) { return {a.x - b.x, a.y - b.y}; }
+__device__ __forceinline__ fxc csub_i(fxc a, fxc b) { return {a.x + b.y, a.y - b.x}; }   // a - i b
+__device__ __forceinline__ fxc cadd_i(fxc a, fxc b) { return {a.x - b.y, a.y + b.x}; }   // a + i b
+
+// z * w / 4 (FULL: z * w), w = (int4){re high, re low, im high, im low} of the
+// 62-bit fixed-point root: low words signed, never -2^31
+template <bool FULL = false>
+__device__ __forceinline__ fxc fx_cmul(fxc z, int4 w) {
+  const int r1 = fx_s1(z.x), r0 = fx_lo(z.x), i1 = fx_s1(z.y), i0 = fx_lo(z.y);
+  const int nz = -w.z, nw = -w.w;
+  constexpr fx half = FULL ? 1LL << 29 : 1LL << 31;
+  const fx m = half + mw(r1, w.y) + mw(r0, w.x) + mw(i1, nw) + mw(i0, nz);
+  const fx n = half + mw(r1, w.w) + mw(r0, w.z) + mw(i1, w.y) + mw(i0, w.x);
+  if constexpr (FULL)
+    return {((mw(r1, w.x) + mw(i1, nz)) << 2) + (m >> 30), ((mw(r1, w.z) + mw(i1, w.x)) << 2) + (n >> 30)};
+  else
+    return {(fx)fx_hi(m) + mw(r1, w.x) + mw(i1, nz), (fx)fx_hi(n) + mw(r1, w.z) + mw(i1, w.x)};
+}
+
+// a * sqrt(1/2) as a - a * (1 - sqrt(1/2)), the factor's 64-bit fraction in two signed words
+__device__ __forceinline__ fx fx_rsqrt2(fx a) {
+  constexpr int c1 = 1257966796, c0 = 102865788;
+  const int a1 = fx_s1(a), a0 = fx_lo(a);
+  const fx m = (1LL << 31) + mw(a1, c0) + mw(a0, c1);
+  return a - ((fx)fx_hi(m) + mw(a1, c1));
+}
+
+__device__ __forceinline__ void fx_dft4(fxc& a0, fxc& a1, fxc& a2, fxc& a3) {
+  const fxc s02 = cadd(a0, a2), d02 = csub(a0, a2), s13 = cadd(a1, a3), d13 = csub(a1, a3);
+  a0 = cadd(s02, s13);
+  a2 = csub(s02, s13);
+  a1 = csub_i(d02, d13);
+  a3 = cadd_i(d02, d13);
+}
+
+template <int R>
+__device__ __forceinline__ void fx_dft(fxc (&x)[R]) {
+  if constexpr (R == 2) {
+    const fxc t = x[0];
+    x[0] = cadd(t, x[1]);
+    x[1] = csub(t, x[1]);
+  } else if constexpr (R == 4) {
+    fx_dft4(x[0], x[1], x[2], x[3]);
+  } else if constexpr (R == 8) {
+    fx_dft4(x[0], x[2], x[4], x[6]);
+    fx_dft4(x[1], x[3], x[5], x[7]);
+    const fxc w1 = {fx_rsqrt2(x[3].x + x[3].y), fx_rsqrt2(x[3].y - x[3].x)};   // W8 x[3]
+    const fxc w3 = {fx_rsqrt2(x[7].y - x[7].x), fx_rsqrt2(x[7].x + x[7].y)};   // conj(W8^3 x[7])
+    const fxc y0 = cadd(x[0], x[1]), y4 = csub(x[0], x[1]);
+    const fxc y1 = cadd(x[2], w1), y5 = csub(x[2], w1);
+    const fxc y2 = csub_i(x[4], x[5]), y6 = cadd_i(x[4], x[5]);
+    const fxc y3 = {x[6].x + w3.x, x[6].y - w3.y}, y7 = {x[6].x - w3.x, x[6].y + w3.y};
+    x[0] = y0, x[1] = y1, x[2] = y2, x[3] = y3, x[4] = y4, x[5] = y5, x[6] = y6, x[7] = y7;
+  }
+}
+
+__device__ __forceinline__ int d_hi(double v) { return __double2hiint(v); }
+
+// The double's value in units of 2^(emax - 1023 - TOP), rounded towards
+// zero; emax: the line's largest biased exponent field
+template <int TOP>
+__device__ __forceinline__ fx fx_from(double v, int emax) {
+  const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
+  const unsigned m = (hi & 0xfffffu) | 0x100000u;
+  const int sh = emax - (int)((hi >> 20) & 0x7ff) + (63 - TOP);
+  unsigned long long u = ((unsigned long long)__funnelshift_l(lo, m, 11) << 32) | (lo << 11);
+  asm("shr.u64 %0, %0, %1;" : "+l"(u) : "r"(sh));   // PTX clamps the amount: zeros and tiny values give 0
+  const fx s = (fx)((int)hi >> 31);
+  return ((fx)u ^ s) - s;
+}
+
+// a * 2^sc as the nearest double (sc << 20 given; no subnormal or overflowing result in the range this form takes)
+__device__ __forceinline__ double fx_to(fx a, int sc20) {
+  const double d = (double)a;
+  const int hi = __double2hiint(d);
+  return __hiloint2double(hi ? hi + sc20 : 0, __double2loint(d));
+}
+
+__device__ __forceinline__ int fx_mag(fxc z) {   // OR of the components' magnitudes, high words
+  const int a = fx_hi(z.x), b = fx_hi(z.y);
+  return (a ^ (a >> 31)) | (b ^ (b >> 31));
+}
+
+// One value per line reduced over the line's threads.  Lines inside one warp
+// in rows mode (and one-thread lines) reduce in registers; others through a
+// shared-memory word per line that the caller zeroed: publish(), a barrier
+// the stages need anyway, read().
+template <int T, int C, bool COLS>
+struct FxLine {
+  static constexpr bool REG = T == 1 || (!COLS && T <= 32);
+  static __device__ __forceinline__ int in_regs_or(int v) {
+    if constexpr (T == 32) return (int)__reduce_or_sync(0xffffffffu, (unsigned)v);
+#pragma unroll
+    for (int o = 1; o < T; o <<= 1) v |= __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+  }
+  static __device__ __forceinline__ int in_regs_max(int v) {
+    if constexpr (T == 32) return __reduce_max_sync(0xffffffffu, v);
+#pragma unroll
+    for (int o = 1; o < T; o <<= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+  }
+  static __device__ __forceinline__ void publish_or(int v, int* slot, int c) {
+    if constexpr (!COLS) {   // one line per warp
+      v = (int)__reduce_or_sync(0xffffffffu, (unsigned)v);
+      if ((threadIdx.x & 31) == 0) atomicOr(slot + c, v);
+    } else {
+      if constexpr (T * C >= 32) {
+#pragma unroll
+        for (int o = C; o < 32; o <<= 1) v |= __shfl_xor_sync(0xffffffffu, v, o);
+        if (C >= 32 || (threadIdx.x & 31) < C) atomicOr(slot + c, v);
+      } else {
+        atomicOr(slot + c, v);
+      }
+    }
+  }
+  static __device__ __forceinline__ void publish_max(int v, int* slot, int c) {
+    if constexpr (!COLS) {
+      v = __reduce_max_sync(0xffffffffu, v);
+      if ((threadIdx.x & 31) == 0) atomicMax(slot + c, v);
+    } else {
+      if constexpr (T * C >= 32) {
+#pragma unroll
+        for (int o = C; o < 32; o <<= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
+        if (C >= 32 || (threadIdx.x & 31) < C) atomicMax(slot + c, v);
+      } else {
+        atomicMax(slot + c, v);
+      }
+    }
+  }
+};
+
+// the shared-memory exchange of line_fft64, its 16-byte elements as integer pairs
+template <int L, int C, bool COLS>
+struct FxSmem {
+  Smem64<L, C, COLS> s;
+  __device__ __forceinline__ void put(int c, int j, fxc v) const {
+    *reinterpret_cast<longlong2*>(s.s + s.idx(c, j)) = make_longlong2(v.x, v.y);
+  }
+  __device__ __forceinline__ fxc get(int c, int j) const {
+    const longlong2 v = *reinterpret_cast<const longlong2*>(s.s + s.idx(c, j));
+    return {v.x, v.y};
+  }
+};
+
+// Shift a line whose magnitudes' OR has high word m to top bit FX_TOP_TW; the exponent follows
+template <int E>
+__device__ __forceinline__ void fx_level(fxc (&v)[E], int m, int& sc) {
+  const int n = __clz(m) - (31 - (FX_TOP_TW - 32));
+  sc -= n;
+  if (n > 0) {
+#pragma unroll
+    for (int e = 0; e < E; e++) v[e] = {v[e].x << n, v[e].y << n};
+  } else if (n < 0) {
+#pragma unroll
+    for (int e = 0; e < E; e++) v[e] = {fx_sar(v[e].x, -n), fx_sar(v[e].y, -n)};
+  }
+}
+
+// the Stockham stages of run_stages64, with the line's exponent carried along
+template <int LOGL, int C, bool COLS, bool WARP_ONLY, int S, class SM>
+__device__ __forceinline__ void fx_stages(fxc (&v)[Sched64<LOGL>::E], int t, int c, const int4* tw, const SM& sm,
+                                          int* slots, int& sc) {
+  using Sc = Sched64<LOGL>;
+  if constexpr (S < Sc::NSTAGES) {
+    constexpr int R = Sc::radix(S), NS = Sc::ns(S), E = Sc::E, T = Sc::T, B = E / R;
+    constexpr bool LAST = S == Sc::NSTAGES - 1;
+    using Ln = FxLine<T, C, COLS>;
+    int mag = 0;
+#pragma unroll
+    for (int u = 0; u < B; u++) {
+      const int b = t + T * u;
+      fxc x[R];
+#pragma unroll
+      for (int r = 0; r < R; r++) x[r] = v[u + B * r];
+      if constexpr (NS > 1) {
+        const int k = b & (NS - 1);
+        x[0] = {fx_sar(x[0].x, 2), fx_sar(x[0].y, 2)};   // the same 1/4 as the products
+#pragma unroll
+        for (int r = 1; r < R; r++) x[r] = fx_cmul(x[r], __ldg(tw + Sc::twoff(S) + (r - 1) * NS + k));
+      }
+      fx_dft<R>(x);
+      if constexpr (LAST) {
+#pragma unroll
+        for (int r = 0; r < R; r++) v[u + B * r] = x[r];
+      } else {
+        const int base = (b / NS) * NS * R + (b & (NS - 1));
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+          mag |= fx_mag(x[r]);
+          sm.put(c, base + r * NS, x[r]);
+        }
+      }
+    }
+    if constexpr (NS > 1) sc += 2;
+    if constexpr (!LAST) {
+      if constexpr (Ln::REG) mag = Ln::in_regs_or(mag);
+      else Ln::publish_or(mag, slots + (S + 1) * C, c);
+      line_sync<WARP_ONLY>();   // this stage's scatter (and the line's magnitudes) are complete
+#pragma unroll
+      for (int e = 0; e < E; e++) v[e] = sm.get(c, t + T * e);
+      if constexpr (!Ln::REG) mag = slots[(S + 1) * C + c];
+      if constexpr (S + 1 < Sc::NSTAGES - 1) line_sync<WARP_ONLY>();   // every gather is done before the next scatter
+      fx_level(v, mag, sc);
+      fx_stages<LOGL, C, COLS, WARP_ONLY, S + 1>(v, t, c, tw, sm, slots, sc);
+    }
+  }
+}
+
+// the FP64 body, for the lines the fixed-point form leaves to it
+template <int LOGL, int C, bool COLS, int KIND, bool TSTORE>
+__device__ __noinline__ void line_fft64_general(const LineParams& p, long long cta) {
+  line_fft64_body<LOGL, C, COLS, KIND, TSTORE>(p, cta);
+}
+
+// The kernel body for one CTA (C lines), arguments as line_fft64_body.
+template <int LOGL, int C, bool COLS, int KIND, bool TSTORE>
+__device__ __forceinline__ void line_fx64_body(const LineParams& p, long long cta) {
+  using Sc = Sched64<LOGL>;
+  constexpr int L = Sc::L, E = Sc::E, T = Sc::T;
+  constexpr bool WARP_ONLY = (!COLS && T <= 32) || (T * C <= 32);
+  using Ln = FxLine<T, C, COLS>;
+  extern __shared__ __align__(1024) double2 smem64[];
+  __shared__ int slots[(Sc::NSTAGES + 1) * C];   // row 0: largest exponents (then the lines' scales), rows 1..: ORs
+  FxSmem<L, C, COLS> sm{{smem64}};
+  const int4* tw = reinterpret_cast<const int4*>(p.tw);
+  const int4* rtw = reinterpret_cast<const int4*>(p.rtw);
+
+  const int tid = threadIdx.x;
+  const int c = COLS ? (tid % C) : (tid / T);
+  const int t = COLS ? (tid / C) : (tid % T);
+  const long long q = cta * C + c;
+  const bool active = q < p.nlines;
+  const long long base = active ? line_off(p.in, q) : 0;
+  // inverse: the forward transform with re and im exchanged on both sides
+  // (not for the C2R loads, whose pre-pass needs them in order)
+  const bool swap = KIND == LK_C2R || (KIND == LK_C2C && p.inverse);
+  const float* in_re = KIND != LK_C2R && swap ? p.in.im : p.in.re;
+  const float* in_im = KIND != LK_C2R && swap ? p.in.re : p.in.im;
+  float* out_re = swap ? p.out.im : p.out.re;
+  float* out_im = swap ? p.out.re : p.out.im;
+
+  double2 d[E];
+#pragma unroll
+  for (int e = 0; e < E; e++) d[e] = make_double2(0.0, 0.0);
+  double dL = 0.0;   // C2R: the real part of bin L (thread 0 of the line)
+  if (active) {
+#pragma unroll
+    for (int e = 0; e < E; e++) {
+      const long long a = base + (long long)(t + T * e) * p.in.es;
+      d[e] = make_double2(ldd(in_re, a), ldd(in_im, a));
+    }
+    if constexpr (KIND == LK_C2R) {
+      if (t == 0) {
+        d[0].y = 0.0;   // bins 0 and L count with their real parts only
+        dL = ldd(p.in.re, base + (long long)L * p.in.es);
+      }
+    }
+  }
+  if constexpr (!Ln::REG) {
+    for (int i = tid; i < (Sc::NSTAGES + 1) * C; i += T * C) slots[i] = 0;
+    line_sync<WARP_ONLY>();
+  }
+  int top = KIND == LK_C2R ? d_hi(dL) & 0x7fffffff : 0;
+#pragma unroll
+  for (int e = 0; e < E; e++) top = max(top, max(d_hi(d[e].x) & 0x7fffffff, d_hi(d[e].y) & 0x7fffffff));
+  // a nonzero top below 2^FX_EXP_MIN: too small, or another thread holds the line's large values; take no chance
+  bool odd = (top >> 20) > FX_EXP_MAX || (top > 0 && (top >> 20) < FX_EXP_MIN);
+  if (top == 0) {   // subnormals too small to show in a high word
+    int low = KIND == LK_C2R ? __double2loint(dL) : 0;
+#pragma unroll
+    for (int e = 0; e < E; e++) low |= __double2loint(d[e].x) | __double2loint(d[e].y);
+    odd = low != 0;
+  }
+  if constexpr (Ln::REG) top = Ln::in_regs_max(top);
+  else Ln::publish_max(top, slots, c);
+  if (__syncthreads_or(odd)) {
+    line_fft64_general<LOGL, C, COLS, KIND, TSTORE>(p, cta);
+    return;
+  }
+  if constexpr (!Ln::REG) top = slots[c];
+  constexpr int TOP = fx_top<LOGL>();
+  const int emax = max(top >> 20, FX_EXP_MIN);   // (a line of zeros: every element shifts out)
+  int sc = emax - 1023 - TOP;
+
+  fxc v[E];
+  if constexpr (KIND == LK_C2R) {
+    // Z'[i] = a - i*b as line_fft64_body, |Z'| up to four times the bins: two bits lower
+    sc += 2;
+#pragma unroll
+    for (int e = 0; e < E; e++) {
+      const int i = t + T * e;
+      const fxc s0 = {fx_from<TOP - 2>(d[e].x, emax), fx_from<TOP - 2>(d[e].y, emax)};
+      fxc z;
+      if (i == 0) {
+        const fx r1 = fx_from<TOP - 2>(dL, emax);
+        z = {s0.x + r1, s0.x - r1};
+      } else {
+        fxc s1 = {0, 0};
+        if (active) {
+          const long long a1 = base + (long long)(L - i) * p.in.es;
+          s1 = {fx_from<TOP - 2>(ldd(p.in.re, a1), emax), fx_from<TOP - 2>(ldd(p.in.im, a1), emax)};
+        }
+        int4 w = __ldg(rtw + i);
+        w.z = -w.z;
+        w.w = -w.w;
+        const fxc a = {s0.x + s1.x, s0.y - s1.y};
+        const fxc b = fx_cmul<true>({s1.x - s0.x, -s1.y - s0.y}, w);
+        z = csub_i(a, b);
+      }
+      v[e] = {z.y, z.x};
+    }
+  } else {
+#pragma unroll
+    for (int e = 0; e < E; e++) {
+      v[e] = {fx_from<TOP>(d[e].x, emax), fx_from<TOP>(d[e].y, emax)};
+    }
+  }
+
+  fx_stages<LOGL, C, COLS, WARP_ONLY, 0>(v, t, c, tw, sm, slots, sc);
+
+  if constexpr (KIND == LK_C2C && TSTORE) {
+    if constexpr (Sc::NSTAGES > 1) __syncthreads();
+#pragma unroll
+    for (int e = 0; e < E; e++) sm.put(c, t + T * e, v[e]);
+    if (t == 0) slots[c] = sc;
+    __syncthreads();
+    const int c2 = tid / T, t2 = tid % T;
+    const long long q2 = cta * C + c2;
+    if (q2 < p.nlines) {
+      const long long ob = line_off(p.out, q2);
+      const int4* twf = reinterpret_cast<const int4*>(p.tw_full);
+      const int r2 = (int)((q2 >> p.tw_qshift) & p.tw_qmask);
+      const int sc20 = (slots[c2] + (p.tw_n ? 2 : 0)) * (1 << 20);
+#pragma unroll
+      for (int e = 0; e < E; e++) {
+        const int k = t2 + T * e;
+        fxc x = sm.get(c2, k);
+        if (p.tw_n) x = fx_cmul(x, __ldg(twf + (long long)r2 * L + k));
+        const long long a = ob + (long long)k * p.out.es;
+        std_(out_re, a, fx_to(x.x, sc20));
+        std_(out_im, a, fx_to(x.y, sc20));
+      }
+    }
+  } else if constexpr (KIND == LK_R2C) {
+    // real forward post-pass as line_fft64_body
+    if constexpr (Sc::NSTAGES > 1) line_sync<WARP_ONLY>();
+#pragma unroll
+    for (int e = 0; e < E; e++) sm.put(c, t + T * e, v[e]);
+    line_sync<WARP_ONLY>();
+    if (active) {
+      const long long ob = line_off(p.out, q);
+      const int sc20 = sc * (1 << 20);
+#pragma unroll
+      for (int e = 0; e < E; e++) {
+        const int k = t + T * e;
+        const fxc s0 = v[e], s1 = sm.get(c, (L - k) & (L - 1));
+        const long long a = ob + (long long)k * p.out.es;
+        if (k == 0) {
+          const long long aL = ob + (long long)L * p.out.es;
+          std_(p.out.re, aL, fx_to(s0.x - s0.y, sc20));
+          std_(p.out.im, aL, 0.0);
+          std_(p.out.re, a, fx_to(s0.x + s0.y, sc20));
+          std_(p.out.im, a, 0.0);
+        } else {
+          const fxc h = {fx_sar(s0.x + s1.x, 1), fx_sar(s0.y - s1.y, 1)};
+          const fxc g = {fx_sar(s0.x - s1.x, 1), fx_sar(s0.y + s1.y, 1)};
+          const fxc x = csub_i(h, fx_cmul<true>(g, __ldg(rtw + k)));
+          std_(p.out.re, a, fx_to(x.x, sc20));
+          std_(p.out.im, a, fx_to(x.y, sc20));
+        }
+      }
+    }
+  } else {
+    if constexpr (KIND == LK_C2C && COLS) {
+      if (p.tw_n) {
+        const int4* twf = reinterpret_cast<const int4*>(p.tw_full);
+        const int r2 = (int)((q >> p.tw_qshift) & p.tw_qmask);
+#pragma unroll
+        for (int e = 0; e < E; e++) v[e] = fx_cmul(v[e], __ldg(twf + (long long)r2 * L + t + T * e));
+        sc += 2;
+      }
+    }
+    if (active) {
+      const long long ob = line_off(p.out, q);
+      const int sc20 = sc * (1 << 20);
+#pragma unroll
+      for (int e = 0; e < E; e++) {
+        const long long a = ob + (long long)(t + T * e) * p.out.es;
+        std_(out_re, a, fx_to(v[e].x, sc20));
+        std_(out_im, a, fx_to(v[e].y, sc20));
+      }
+    }
+  }
+}
+
+// 1024 resident threads (64 registers each): at the 80 to 120 registers the
+// compiler takes on its own, 4096-point lines have one CTA per SM and no
+// other's work under its barriers (4096 x 4096 c2c 0.346 vs 0.259 ms, 512^3-
+// point real volumes 3% slower); 1280 threads spill (256-point lines 0.156 vs 0.171 ms)
+template <int LOGL, int C, bool COLS, int KIND, bool TSTORE>
+__global__ void __launch_bounds__(Sched64<LOGL>::T * C, 1024 / (Sched64<LOGL>::T * C)) line_fx64(const LineParams p) {
+  line_fx64_body<LOGL, C, COLS, KIND, TSTORE>(p, blockIdx.x);
+}
+
+}  // namespace agb

@@ -20,6 +20,7 @@
 //    through scratch).
 #include <cuda_fp16.h>
 
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -90,7 +91,7 @@ static TableCache& tcache() {
 }
 
 // Device copy of table (type, key) on the current device; `make` builds the
-// host table (a std::vector of float2 or double2) on the first request only.
+// host table (a std::vector of float2 or int4) on the first request only.
 template <class F>
 static auto cached_table(int type, long long key, F make) -> const typename decltype(make())::value_type* {
   using V = typename decltype(make())::value_type;
@@ -263,17 +264,31 @@ const float2* fourstep_full_table(long long N, long long L2) {
   return cached_table(4, (N << 6) | l2, [&] { return fourstep_full_table_host(N, L2); });
 }
 
-// FP64 tables: the same roots without the rounding to FP32
-static double2 root_d(long long m, long long N) {
+// FP64 tables: the same roots in 62-bit fixed point, each component as high *
+// 2^32 + low with a signed low word (never -2^31: the kernels negate it).
+// The FP64 value's own error (2^-54) is the larger one.
+static void split62(double v, int* hi, int* lo) {
+  const long long w = std::llrint(std::ldexp(v, 62));
+  *hi = (int)((w + (1LL << 31)) >> 32);
+  *lo = (int)(w - (long long)*hi * (1LL << 32));
+  if (*lo == INT_MIN) *lo += 1;
+  // +-1 exactly: one unit (2^-62) nearer to zero, so that the products' exact
+  // quarters round their ties by the sign of the data and leave no mean
+  if (*lo == 0 && *hi != 0) *lo = *hi > 0 ? -1 : 1;
+}
+static int4 root_d(long long m, long long N) {
   double c, s;
   unit_root(m, N, &c, &s);
-  return make_double2(c, s);
+  int4 w;
+  split62(c, &w.x, &w.y);
+  split62(s, &w.z, &w.w);
+  return w;
 }
 
 template <int LOGL>
-static std::vector<double2> stage_table64() {
+static std::vector<int4> stage_table64() {
   using S = Sched64<LOGL>;
-  std::vector<double2> t(S::twsize());
+  std::vector<int4> t(S::twsize());
   for (int s = 0; s < S::NSTAGES; s++) {
     int ns = S::ns(s), R = S::radix(s);
     if (ns == 1) continue;
@@ -285,34 +300,34 @@ static std::vector<double2> stage_table64() {
 }
 
 template <int... Ls>
-static std::vector<double2> stage_table64_dispatch(int logl, std::integer_sequence<int, Ls...>) {
-  std::vector<double2> out;
+static std::vector<int4> stage_table64_dispatch(int logl, std::integer_sequence<int, Ls...>) {
+  std::vector<int4> out;
   ((logl == Ls ? (void)(out = stage_table64<Ls>()) : (void)0), ...);
   return out;
 }
 
-std::vector<double2> stage_table64_host(int logl) {
+std::vector<int4> stage_table64_host(int logl) {
   return stage_table64_dispatch(logl, std::make_integer_sequence<int, ROWS_MAX_LOG64 + 1>{});
 }
 
-const double2* stage_twiddles64(int logl) {
+const int4* stage_twiddles64(int logl) {
   return cached_table(5, logl, [&] { return stage_table64_host(logl); });
 }
 
-const double2* real_twiddles64(long long L) {
+const int4* real_twiddles64(long long L) {
   return cached_table(6, L, [&] {
-    std::vector<double2> t(L);
+    std::vector<int4> t(L);
     for (long long k = 0; k < L; k++) t[k] = root_d(k, 2 * L);
     return t;
   });
 }
 
-const double2* fourstep_full_table64(long long N, long long L2) {
+const int4* fourstep_full_table64(long long N, long long L2) {
   int l2 = 0;
   while ((1LL << l2) < L2) l2++;
   return cached_table(7, (N << 6) | l2, [&] {
     const long long L1 = N / L2;
-    std::vector<double2> t(N);
+    std::vector<int4> t(N);
     for (long long j = 0; j < L2; j++)
       for (long long k = 0; k < L1; k++) t[j * L1 + k] = root_d(j * k, N);
     return t;
@@ -557,7 +572,7 @@ struct Builder {
         P.has_tma = true;
       }
       if (f64) {
-        // the FP64 kernels read double2 tables through the same fields
+        // the FP64 kernels read int4 tables through the same fields
         op.p.tw = reinterpret_cast<const float2*>(stage_twiddles64(op.k.stage_logl));
         if (tw_n) op.p.tw_full = reinterpret_cast<const float2*>(fourstep_full_table64(tw_n, tw_qmask + 1));
         if (real_L) op.p.rtw = reinterpret_cast<const float2*>(real_twiddles64(real_L));

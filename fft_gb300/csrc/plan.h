@@ -160,13 +160,13 @@ void fourstep_tables(long long N, const float2** hi, const float2** lo, int* lo_
 #endif
 constexpr long long kFullTableMax = 1LL << AFFT_FULL_TABLE_LOG;
 const float2* fourstep_full_table(long long N, long long L2);
-// FP64 tables (computed in FP64, no rounding): stage twiddles of the FP64
+// FP64 tables (computed in FP64, kept in 62-bit fixed point): stage twiddles of the FP64
 // line kernels, W_{2L}^k (k < L), and the four-step matrix W_N^{t2 k} at
 // [t2 * L1 + k] for any N
-const double2* stage_twiddles64(int logl);
-const double2* real_twiddles64(long long L);
-const double2* fourstep_full_table64(long long N, long long L2);
-std::vector<double2> stage_table64_host(int logl);
+const int4* stage_twiddles64(int logl);
+const int4* real_twiddles64(long long L);
+const int4* fourstep_full_table64(long long N, long long L2);
+std::vector<int4> stage_table64_host(int logl);
 std::vector<float2> fourstep_full_table_host(long long N, long long L2);
 // The same tables on the host, without touching the device.
 std::vector<float2> stage_table_host(int logl);
