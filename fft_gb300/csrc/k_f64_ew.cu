@@ -28,6 +28,7 @@ __device__ __forceinline__ double ld64(const float* base, long long off) {
 }  // namespace
 
 __global__ void real_pass_kernel64(const RealPassParams p) {
+  pdl_enter();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long half = p.L / 2 + 1;
   long long q, k;
@@ -82,6 +83,7 @@ __global__ void real_pass_kernel64(const RealPassParams p) {
 }
 
 __global__ void copy_lines_kernel64(const CopyParams p) {
+  pdl_enter();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= p.nlines * p.len) return;
   const long long q = idx / p.len, i = idx - q * p.len;
@@ -92,6 +94,7 @@ __global__ void copy_lines_kernel64(const CopyParams p) {
 }
 
 __global__ void real1_kernel64(const RealPassParams p) {
+  pdl_enter();
   const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= p.nlines) return;
   const long long i = line_off(p.in, q), o = line_off(p.out, q);

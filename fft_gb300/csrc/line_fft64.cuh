@@ -196,7 +196,7 @@ __device__ __forceinline__ void run_stages64(double2 (&v)[Sched64<LOGL>::E], int
 }
 
 __device__ __forceinline__ double ldd(const float* base, long long off) {
-  return __ldg(reinterpret_cast<const double*>(base) + off);
+  return ldin(reinterpret_cast<const double*>(base) + off);
 }
 __device__ __forceinline__ void std_(float* base, long long off, double v) {
   reinterpret_cast<double*>(base)[off] = v;
@@ -354,6 +354,7 @@ __device__ __forceinline__ void line_fft64_body(const LineParams& p, long long c
 
 template <int LOGL, int C, bool COLS, int KIND, bool TSTORE>
 __global__ void __launch_bounds__(Sched64<LOGL>::T * C) line_fft64(const LineParams p) {
+  pdl_enter();
   line_fft64_body<LOGL, C, COLS, KIND, TSTORE>(p, blockIdx.x);
 }
 

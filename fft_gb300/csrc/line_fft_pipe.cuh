@@ -296,7 +296,7 @@ __device__ __forceinline__ void pipe_loop(long long first, long long ntiles, uin
       float2 bl = make_float2(0.f, 0.f);
       if (t == 0) {
         const long long oL = line_off(p.in, q) + (long long)L * p.in.es;
-        bl = make_float2(__ldg(p.in.re + oL), __ldg(p.in.im + oL));
+        bl = make_float2(ldin(p.in.re + oL), ldin(p.in.im + oL));
       }
 #pragma unroll
       for (int e = 0; e < E; e++) {
@@ -477,6 +477,7 @@ line_fft_pipe(const __grid_constant__ LineParams p, const __grid_constant__ TmaT
   extern __shared__ __align__(1024) float2 smem_raw[];
   float* raw = reinterpret_cast<float*>(smem_raw);
   const uint32_t mb = smem_u32(&mbar), raw_s = smem_u32(raw);
+  pdl_enter();
   pipe_loop<LOGL, C, KIND, pipe_bulk<LOGL, KIND>() && !TSTORE, TSTORE>(
       blockIdx.x, ntiles, mb, raw, raw + 2 * Sched<LOGL>::L * C, &tmo,
       [&](long long tile, long long* cta) -> const LineParams& {
@@ -525,6 +526,7 @@ line_fft_tma_bulk(const __grid_constant__ LineParams p, const __grid_constant__ 
   constexpr int L = Sched<LOGL>::L;
   __shared__ __align__(8) uint64_t mbar;
   extern __shared__ __align__(1024) float2 smem_raw[];
+  pdl_enter();
   if (!tma_load_tile<C>(p, tm, blockIdx.x, &mbar, smem_raw)) return;
   line_fft_body<LOGL, C, true, KIND, false, false, 0, true, true>(p, blockIdx.x);
   if (threadIdx.x == 0) {

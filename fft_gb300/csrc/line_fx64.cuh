@@ -466,6 +466,7 @@ __device__ __forceinline__ void line_fx64_body(const LineParams& p, long long ct
 // point real volumes 3% slower); 1280 threads spill (256-point lines 0.156 vs 0.171 ms)
 template <int LOGL, int C, bool COLS, int KIND, bool TSTORE>
 __global__ void __launch_bounds__(Sched64<LOGL>::T * C, 1024 / (Sched64<LOGL>::T * C)) line_fx64(const LineParams p) {
+  pdl_enter();
   line_fx64_body<LOGL, C, COLS, KIND, TSTORE>(p, blockIdx.x);
 }
 

@@ -1176,6 +1176,25 @@ bool op_tables_ok(const Op& op) {
          (!op.k.plane_log1 || op.p.tw2);
 }
 
+// One launch of a plan.  Programmatic stream serialization: the kernel may
+// start while the launch before it drains (it waits for that one's results in
+// pdl_enter before touching any array).
+template <class... P>
+static void launch_pass(void (*fn)(P...), long long grid, int threads, size_t smem, cudaStream_t st,
+                        const std::common_type_t<P>&... args) {
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  (void)cudaLaunchKernelEx(&cfg, fn, args...);   // an error stays for launch()'s check of the last one
+}
+
 int Plan::launch(const float* src_re, const float* src_im, float* dst_re, float* dst_im, cudaStream_t st) {
   if (scratch_elems > 0 && !scratch) {
     if (cudaMalloc(&scratch, (size_t)scratch_elems * esize()) != cudaSuccess) {
@@ -1207,7 +1226,7 @@ int Plan::launch(const float* src_re, const float* src_im, float* dst_re, float*
       // costs more, 2048² c2r 0.0324 vs 0.0300 ms)
       const long long slots = (long long)sm_count * op.k.pipe_ctas;
       if (op.k.paired_tma && tma_paired(p, op.k, &pt)) {
-        op.k.paired_tma<<<(unsigned)op.grid, op.threads, op.k.paired_smem, st>>>(p, pt);
+        launch_pass(op.k.paired_tma, op.grid, op.threads, op.k.paired_smem, st, p, pt);
       } else if (op.k.pipe && sm_count > 0 && (op.k.logl == 11 || op.grid >= 2 * slots) && tma_tile(p, op.k, &tm) &&
           (!(AFFT_PIPE_BULK_STORE && !op.k.tstore &&
              ((op.k.kind == LK_C2C && (op.k.logl == 11 || AFFT_PIPE_BULK10)) ||
@@ -1215,32 +1234,29 @@ int Plan::launch(const float* src_re, const float* src_im, float* dst_re, float*
            tma_tile_out(p, op.k, &tmo))) {
         // persistent: at most pipe_ctas CTAs per SM, each walking tiles gridDim.x apart
         const long long g = std::min<long long>(op.grid, slots);
-        op.k.pipe<<<(unsigned)g, op.threads, op.k.pipe_smem, st>>>(p, tm, tmo, op.grid);
+        launch_pass(op.k.pipe, g, op.threads, op.k.pipe_smem, st, p, tm, tmo, op.grid);
       } else if (op.k.tma_bulk && tma_tile(p, op.k, &tm) && tma_tile_out(p, op.k, &tmo)) {
-        op.k.tma_bulk<<<(unsigned)op.grid, op.threads, op.smem, st>>>(p, tm, tmo);
+        launch_pass(op.k.tma_bulk, op.grid, op.threads, op.smem, st, p, tm, tmo);
       } else if (op.k.tma && tma_tile(p, op.k, &tm)) {
-        op.k.tma<<<(unsigned)op.grid, op.threads, op.smem, st>>>(p, tm);
+        launch_pass(op.k.tma, op.grid, op.threads, op.smem, st, p, tm);
       } else {
-        op.k.fn<<<(unsigned)op.grid, op.threads, op.smem, st>>>(p);
+        launch_pass(op.k.fn, op.grid, op.threads, op.smem, st, p);
       }
     } else if (op.type == OP_REAL) {
       RealPassParams rp = op.rp;
       rp.in = bind(op.in, base, esz);
       rp.out = bind(op.out, base, esz);
-      if (dbl) real_pass_kernel64<<<(unsigned)op.grid, op.threads, 0, st>>>(rp);
-      else real_pass_kernel<<<(unsigned)op.grid, op.threads, 0, st>>>(rp);
+      launch_pass(dbl ? real_pass_kernel64 : real_pass_kernel, op.grid, op.threads, 0, st, rp);
     } else if (op.type == OP_COPY) {
       CopyParams cp = op.cp;
       cp.in = bind(op.in, base, esz);
       cp.out = bind(op.out, base, esz);
-      if (dbl) copy_lines_kernel64<<<(unsigned)op.grid, op.threads, 0, st>>>(cp);
-      else copy_lines_kernel<<<(unsigned)op.grid, op.threads, 0, st>>>(cp);
+      launch_pass(dbl ? copy_lines_kernel64 : copy_lines_kernel, op.grid, op.threads, 0, st, cp);
     } else {
       RealPassParams rp = op.rp;
       rp.in = bind(op.in, base, esz);
       rp.out = bind(op.out, base, esz);
-      if (dbl) real1_kernel64<<<(unsigned)op.grid, op.threads, 0, st>>>(rp);
-      else real1_kernel<<<(unsigned)op.grid, op.threads, 0, st>>>(rp);
+      launch_pass(dbl ? real1_kernel64 : real1_kernel, op.grid, op.threads, 0, st, rp);
     }
   }
   cudaError_t e = cudaGetLastError();

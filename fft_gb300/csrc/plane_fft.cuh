@@ -92,15 +92,15 @@ __device__ __forceinline__ void plane_body(const LineParams& p, long long cta) {
         const float* pr = p.in.re + bin + r * D2 + t;
         const float* pi = p.in.im + bin + r * D2 + t;
 #pragma unroll
-        for (int e = 0; e < E; e++) v[e] = make_float2(__ldg(pr + T2 * e), __ldg(pi + T2 * e));
+        for (int e = 0; e < E; e++) v[e] = make_float2(ldin(pr + T2 * e), ldin(pi + T2 * e));
       } else {
         const float* pz = p.in.re + bin + 2 * (r * D2 + t);
         if (!(reinterpret_cast<uintptr_t>(pz) & 7)) {
 #pragma unroll
-          for (int e = 0; e < E; e++) v[e] = __ldg(reinterpret_cast<const float2*>(pz) + T2 * e);
+          for (int e = 0; e < E; e++) v[e] = ldin(reinterpret_cast<const float2*>(pz) + T2 * e);
         } else {
 #pragma unroll
-          for (int e = 0; e < E; e++) v[e] = make_float2(__ldg(pz + 2 * T2 * e), __ldg(pz + 2 * T2 * e + 1));
+          for (int e = 0; e < E; e++) v[e] = make_float2(ldin(pz + 2 * T2 * e), ldin(pz + 2 * T2 * e + 1));
         }
       }
     } else {
@@ -165,6 +165,7 @@ __device__ __forceinline__ void plane_body(const LineParams& p, long long cta) {
 template <int LOG1, int LOG2, int UNIT>
 __global__ void __launch_bounds__(PlaneShape<LOG1, LOG2>::NT, min_ctas<PlaneShape<LOG1, LOG2>::NT>())
 plane_fft(const LineParams p) {
+  pdl_enter();
   plane_body<LOG1, LOG2, UNIT>(p, blockIdx.x);
 }
 

@@ -97,14 +97,17 @@ __device__ __forceinline__ void real1_body(const RealPassParams& p, long long q)
 }
 
 __global__ void real_pass_kernel(const RealPassParams p) {
+  pdl_enter();
   real_pass_body(p, (long long)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 __global__ void copy_lines_kernel(const CopyParams p) {
+  pdl_enter();
   copy_body(p, (long long)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 __global__ void real1_kernel(const RealPassParams p) {
+  pdl_enter();
   real1_body(p, (long long)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
