@@ -295,17 +295,17 @@ __device__ __forceinline__ long long line_off(const LineIO& io, long long q) {
 __device__ __forceinline__ float2 ldg2(const float2* p) { return __ldg(p); }
 
 // Start of a kernel that a plan launches with programmatic stream
-// serialization: once every CTA of this grid is resident or done, the next
-// launch's CTAs may take the free slots, and nothing before this point
-// depends on the previous launch, which is complete and visible after it.
-// The last wave of one pass then hides the launch and the start of the next:
-// 256^3 c2c (three passes) 133.6 -> 125.8 us a transform, 37 images of 512^2
-// 68.9 -> 63.8, 30011 real lines of 512 points 27.9 -> 25.3, 16384 lines of
-// 4096 points 174.2 -> 171.7, 128x128x256 x 2 real FP64 there and back 297 -> 281.
-__device__ __forceinline__ void pdl_enter() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-}
+// serialization: once every CTA of the previous launch has ended or is in its
+// last wave's drain, this grid's CTAs may take the free slots; they wait here
+// until that launch is complete and its results are visible.  The drain of
+// one pass then hides the launch and the start of the next: 256^3 c2c (three
+// passes) 133.6 -> 125.8 us a transform, 37 images of 512^2 68.9 -> 63.8,
+// 30011 real lines of 512 points 27.9 -> 25.3, 16384 lines of 4096 points
+// 174.2 -> 171.7, 128x128x256 x 2 real FP64 there and back 297 -> 281.  (No
+// explicit launch_dependents: it gains nothing over the trigger at each CTA's
+// end, and costs passes of many small CTAs 1.6 times their time, 2 x 1024
+// x 6895 c2c 154 -> 262.)
+__device__ __forceinline__ void pdl_enter() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Loads of the arrays a pass transforms.  Coherent ones: the previous launch
 // may still be writing them while this grid's CTAs start (pdl_enter), which
