@@ -8,10 +8,10 @@
 // each group is ONE launch (line_fft_grouped or elementwise_grouped) of one
 // CTA per virtual CTA, which finds its segment in a per-virtual-CTA map.
 // The first run builds a CUDA graph with one kernel node per group, which
-// depends on exactly the groups that ran the previous pass of its own
-// transforms (the transforms are independent of each other), so a pass of
-// one transform starts as soon as its own previous pass has finished; later
-// runs replay the graph.
+// depends on the groups that ran the previous pass of its own transforms
+// (the transforms are independent of each other) and on the group before it
+// on one of kQueueLanes lanes, so a pass of one transform starts about as
+// soon as its own previous pass has finished; later runs replay the graph.
 //
 // Scratch for transforms whose plans need it (four-step passes, real
 // inverse of N-D arrays) comes from one queue-owned arena, a disjoint region
@@ -305,9 +305,30 @@ static int build_queue(QueueImpl& Q) {
   return 0;
 }
 
+// Graph branches the groups are spread over.  A graph as wide as the groups'
+// own dependencies allow (50 to 100 branches) costs the device several
+// hundred us of set-up per launch when it comes behind another graph's: 245
+// mixed transforms took 723 us a run in rotation with two other queues and
+// 290 us alone.  With 12 branches 290 us either way (60 transforms 253 -> 104,
+// 1000 transforms 1620 -> 1230, 3000 3430 before and after); 8 and 16
+// branches within 10% of that, 32 up to twice as slow, 1 (a chain) 780 us.
+constexpr int kQueueLanes = 12;
+
 static int capture(QueueImpl& Q) {
   // one node per group (an empty node for a group without work, so the
   // dependency chain stays whole), with edges from its predecessor groups
+  // and from the group before it on its lane: each group goes to the lane
+  // with the least work so far, counted in threads, at least one full wave
+  // (a small group takes its latency all the same)
+  int sms = 0;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, Q.device) != cudaSuccess) {
+    cudaGetLastError();
+    sms = 1;
+  }
+  const long long wave = (long long)sms * 2048;
+  long long load[kQueueLanes] = {};
+  int last[kQueueLanes];
+  std::fill(last, last + kQueueLanes, -1);
   cudaGraph_t graph = nullptr;
   if (cudaGraphCreate(&graph, 0) != cudaSuccess) return AFFT_GB300_ECUDA;
   std::vector<cudaGraphNode_t> node(Q.groups.size());
@@ -315,7 +336,12 @@ static int capture(QueueImpl& Q) {
   for (size_t n = 0; n < Q.groups.size() && ok; n++) {
     Group& g = Q.groups[n];
     std::vector<cudaGraphNode_t> deps;
-    for (int p : g.preds) deps.push_back(node[p]);
+    const int lane = (int)(std::min_element(load, load + kQueueLanes) - load);
+    for (int p : g.preds)
+      if (p != last[lane]) deps.push_back(node[p]);
+    if (last[lane] >= 0) deps.push_back(node[last[lane]]);
+    last[lane] = (int)n;
+    load[lane] += std::max(wave, g.total * g.threads);
     if (g.total == 0) {
       ok = cudaGraphAddEmptyNode(&node[n], graph, deps.data(), deps.size()) == cudaSuccess;
       continue;
