@@ -108,9 +108,9 @@ def last_error():
 
 
 def _check(what):
-    code, msg = last_error()
+    code = lib().afft_gb300_last_error()
     if code:
-        raise AfftError("%s: %s (%s)" % (what, msg, ERRORS.get(code, code)))
+        raise AfftError("%s: %s (%s)" % (what, last_error()[1], ERRORS.get(code, code)))
 
 
 def alignment():
@@ -131,18 +131,32 @@ def ptr(a):
         return None
     if isinstance(a, int):
         return a
-    if hasattr(a, "data_ptr"):
-        return a.data_ptr()
+    f = getattr(a, "data_ptr", None)
+    if f is not None:
+        return f()
+    f = getattr(a, "__array_interface__", None)   # numpy: a quarter of the time of a.ctypes.data
+    if f is not None:
+        return f["data"][0]
     if hasattr(a, "ctypes"):
         return a.ctypes.data
     raise TypeError(type(a))
 
 
-def _validate(kind, dims, batch, fmt, bits, src_re, src_im, dst_re, dst_im):
-    """Check the array objects a transform call gets (numpy arrays, torch
-    tensors): element type, contiguity and size against what the transform
-    reads and writes, so that a wrong array is refused here instead of the
-    kernels reading or writing past it.  Raw int pointers are not checked."""
+_ROLES = ("src_re", "src_im", "dst_re", "dst_im")
+_FLOAT_DTYPES = {}   # torch and numpy dtypes seen so far that are float32 or float64 -> their names
+
+
+def _dtype_name(dtype):
+    name = _FLOAT_DTYPES.get(dtype)
+    if name is None:
+        name = str(dtype).split(".")[-1]
+        if name in ("float32", "float64"):
+            _FLOAT_DTYPES[dtype] = name
+    return name
+
+
+def _wants(kind, dims, batch, fmt):
+    """Elements a transform reads or writes of each array of _ROLES (0: none)."""
     k = KINDS[kind] if isinstance(kind, str) else kind
     d = squeeze(dims)
     n = 1
@@ -153,20 +167,31 @@ def _validate(kind, dims, batch, fmt, bits, src_re, src_im, dst_re, dst_im):
     cin, cout = k != KIND_R, k != KIND_RI
     m_in = (h if k == KIND_RI else n) * batch
     m_out = (h if k == KIND_R else n) * batch
-    want = {"src_re": m_in * (2 if cin and inter else 1), "src_im": m_in if cin and not inter else 0,
-            "dst_re": m_out * (2 if cout and inter else 1), "dst_im": m_out if cout and not inter else 0}
-    name = "float64" if bits == 64 else "float32"
-    for role, a in (("src_re", src_re), ("src_im", src_im), ("dst_re", dst_re), ("dst_im", dst_im)):
-        if a is None or isinstance(a, int) or not want[role] or not hasattr(a, "dtype"):
+    return (m_in * (2 if cin and inter else 1), m_in if cin and not inter else 0,
+            m_out * (2 if cout and inter else 1), m_out if cout and not inter else 0)
+
+
+def _check_arrays(wants, name, arrays):
+    for want, a, role in zip(wants, arrays, _ROLES):
+        if not want or a is None or isinstance(a, int) or not hasattr(a, "dtype"):
             continue
-        if str(a.dtype).split(".")[-1] != name:
+        if _dtype_name(a.dtype) != name:
             raise AfftError("%s: %s array expected, got %s" % (role, name, a.dtype))
         size = a.numel() if hasattr(a, "numel") else a.size
         contig = a.is_contiguous() if hasattr(a, "is_contiguous") else a.flags["C_CONTIGUOUS"]
         if not contig:
             raise AfftError("%s: the array must be contiguous" % role)
-        if size < want[role]:
-            raise AfftError("%s: %d elements, the transform needs %d" % (role, size, want[role]))
+        if size < want:
+            raise AfftError("%s: %d elements, the transform needs %d" % (role, size, want))
+
+
+def _validate(kind, dims, batch, fmt, bits, src_re, src_im, dst_re, dst_im):
+    """Check the array objects a transform call gets (numpy arrays, torch
+    tensors): element type, contiguity and size against what the transform
+    reads and writes, so that a wrong array is refused here instead of the
+    kernels reading or writing past it.  Raw int pointers are not checked."""
+    _check_arrays(_wants(kind, dims, batch, fmt), "float64" if bits == 64 else "float32",
+                  (src_re, src_im, dst_re, dst_im))
 
 
 def describe(kind, dims, batch=1, fmt=0):
@@ -282,6 +307,8 @@ class _Plan:
             _check("create")
             raise AfftError("create failed")
         self._fn = getattr(L, "afft_%d_%s_transform" % (bits, name))
+        self._want = _wants(self.kind, self.dims, 1, fmt)
+        self._dtype = "float%d" % bits
 
     def __bool__(self):
         return bool(self.state)
@@ -307,7 +334,7 @@ class complex_transform(_Plan):
     kind = KIND_C
 
     def __call__(self, src_re, src_im, dst_re, dst_im):
-        _validate(self.kind, self.dims, 1, self.format, self.bits, src_re, src_im, dst_re, dst_im)
+        _check_arrays(self._want, self._dtype, (src_re, src_im, dst_re, dst_im))
         self._fn(self.state, ptr(src_re), ptr(src_im), ptr(dst_re), ptr(dst_im))
         _check("transform")
 
@@ -322,7 +349,7 @@ class real_transform(_Plan):
     kind = KIND_R
 
     def __call__(self, src, dst_re, dst_im):
-        _validate(self.kind, self.dims, 1, self.format, self.bits, src, None, dst_re, dst_im)
+        _check_arrays(self._want, self._dtype, (src, None, dst_re, dst_im))
         self._fn(self.state, ptr(src), ptr(dst_re), ptr(dst_im))
         _check("transform")
 
@@ -332,7 +359,7 @@ class inverse_real_transform(_Plan):
     kind = KIND_RI
 
     def __call__(self, src_re, src_im, dst):
-        _validate(self.kind, self.dims, 1, self.format, self.bits, src_re, src_im, dst, None)
+        _check_arrays(self._want, self._dtype, (src_re, src_im, dst, None))
         self._fn(self.state, ptr(src_re), ptr(src_im), ptr(dst))
         _check("transform")
 
@@ -372,17 +399,16 @@ class BatchPlan:
             raise AfftError("batch_create failed")
         name = {KIND_C: "c", KIND_CI: "ci", KIND_R: "r", KIND_RI: "ri"}[self.kind]
         self._fn = getattr(L, "afft_%d_%s_transform" % (64 if form == "f64" else 32, name))
+        self._launch = L.afft_gb300_transform_async
+        self._want = _wants(self.kind, self.dims, self.batch, self.format)
+        self._dtype = "float64" if form == "f64" else "float32"
 
     def __call__(self, a, b=None, c=None, d=None):
-        bits = 64 if self.form == "f64" else 32
         if self.kind in (KIND_C, KIND_CI):
-            _validate(self.kind, self.dims, self.batch, self.format, bits, a, b, c, d)
+            _check_arrays(self._want, self._dtype, (a, b, c, d))
             self._fn(self.state, ptr(a), ptr(b), ptr(c), ptr(d))
-        elif self.kind == KIND_R:
-            _validate(self.kind, self.dims, self.batch, self.format, bits, a, None, b, c)
-            self._fn(self.state, ptr(a), ptr(b), ptr(c))
         else:
-            _validate(self.kind, self.dims, self.batch, self.format, bits, a, b, c, None)
+            _check_arrays(self._want, self._dtype, (a, None, b, c) if self.kind == KIND_R else (a, b, c, None))
             self._fn(self.state, ptr(a), ptr(b), ptr(c))
         _check("transform")
 
@@ -390,10 +416,8 @@ class BatchPlan:
         """Enqueue without waiting; ``stream`` is a torch.cuda.Stream, a raw
         cudaStream_t int, or None for the CUDA default stream."""
         s = stream.cuda_stream if hasattr(stream, "cuda_stream") else stream
-        _validate(self.kind, self.dims, self.batch, self.format, 64 if self.form == "f64" else 32,
-                  src_re, src_im, dst_re, dst_im)
-        rc = lib().afft_gb300_transform_async(self.state, ptr(src_re), ptr(src_im), ptr(dst_re), ptr(dst_im), s)
-        if rc:
+        _check_arrays(self._want, self._dtype, (src_re, src_im, dst_re, dst_im))
+        if self._launch(self.state, ptr(src_re), ptr(src_im), ptr(dst_re), ptr(dst_im), s):
             _check("transform_async")
 
     @property

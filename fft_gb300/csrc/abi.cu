@@ -273,13 +273,14 @@ static void io_elems(const Plan& P, long long* in_n, long long* out_n) {
 
 // A kernel whose bounded wait gave up (a TC-form kernel waiting for its
 // tensor-core results: 1; a cols pass waiting for its TMA-loaded tile: 2)
-// sets the device error word instead of hanging; report and clear it.
+// sets the device's error word instead of hanging; report and clear it (after
+// the stream's synchronize).
 static int check_tc_error(const Plan& P) {
   if (P.form != FORM_TC && !P.has_tma) return 0;
-  int* w = tc_error_word();
-  int v = 0;
-  if (w && cudaMemcpy(&v, w, sizeof(int), cudaMemcpyDeviceToHost) == cudaSuccess && v) {
-    cudaMemset(w, 0, sizeof(int));
+  volatile int* w = tc_error_word();
+  const int v = w ? *w : 0;
+  if (v) {
+    *w = 0;
     set_error(AFFT_GB300_ETIMEOUT, v == 2 ? "TMA tile wait timed out" : "tensor-core stage wait timed out");
     return AFFT_GB300_ETIMEOUT;
   }
