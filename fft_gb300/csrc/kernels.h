@@ -132,13 +132,13 @@ bool get_cols_real(int logl, int kind, LineKernel* out);
 // segments are the floor).  Complex 512-point cols passes take 8 lines
 // (32 KB tiles, 4 CTAs per SM): 4-6% faster for four-step 2^17/2^18 axes;
 // the real 512-point cols passes measured 7% slower that way and keep 16.
-#ifndef AFFT_SMALLC
-#define AFFT_SMALLC 4
-#endif
+// Up to 16 points a line is one thread: 256 lines, 256 threads (with 32, CTAs
+// of one warp, 2 x 1024 x 6895 c2c took 154 instead of 79 us; 32- and 64-point
+// lines gain nothing from more than 32).
 template <int LOGL, bool COLS>
 constexpr int lines_per_cta() {
   constexpr int T = Sched<LOGL>::T;
-  if constexpr (COLS) return LOGL <= AFFT_SMALLC ? 256 / T : LOGL <= 7 ? 32 : (LOGL <= 9 ? 16 : 8);
+  if constexpr (COLS) return LOGL <= 4 ? 256 / T : LOGL <= 7 ? 32 : (LOGL <= 9 ? 16 : 8);
   else return T >= 256 ? 1 : 256 / T;
 }
 
