@@ -26,9 +26,9 @@
 //
 // Bounds, in bits (component magnitudes; |z| is the complex magnitude): first
 // stage's output |z| < 2^62.5, every intermediate < 2^63; before a twiddle
-// product the line is shifted so that its top bit is bit 59 (components
-// < 2^60, |z| < 2^60.5); the product is scaled by 1/4: |z| < 2^58.5, and
-// < 2^61.5 after the next radix-8 stage.
+// product the line's top bit is bit 57 to 60 (59 before the last stage of a
+// real forward pass; components < 2^61, |z| < 2^61.5); the product is scaled
+// by 1/4: |z| < 2^59.5, and < 2^62.5 after the next radix-8 stage.
 #pragma once
 
 #include "line_fft64.cuh"
@@ -49,7 +49,9 @@ constexpr int fx_top() {
   using Sc = Sched64<LOGL>;
   return Sc::FIRST == 2 ? 60 : Sc::FIRST == 4 ? 59 : Sc::NSTAGES > 1 ? 58 : 57;
 }
-constexpr int FX_TOP_TW = 59;     // the same where a twiddle product follows
+constexpr int FX_TOP_TW = 59;     // the same where a twiddle product follows, when shifted there
+constexpr int FX_TOP_MIN = 57, FX_TOP_MAX = 60;   // and where it is left as it is (59 before the last stage of
+                                                  // a pass that adds its output in pairs, the real forward)
 constexpr int FX_EXP_MIN = 200;   // biased exponents the fixed-point form takes: below, subnormal results are
 constexpr int FX_EXP_MAX = 2000;  // possible; above, overflow (14 bits of growth) and non-finite values
 
@@ -58,7 +60,6 @@ __device__ __forceinline__ int fx_lo(fx a) { return (int)a; }
 // a = fx_s1(a) * 2^32 + (signed) fx_lo(a)
 __device__ __forceinline__ int fx_s1(fx a) { return fx_hi(a) + (int)((unsigned)fx_lo(a) >> 31); }
 __device__ __forceinline__ fx mw(int a, int b) { return (fx)a * (fx)b; }
-
 // a / 2^n to nearest, ties away from zero: a mean of half a tie would add up
 // over a line to an error in bin 0
 __device__ __forceinline__ fx fx_sar(fx a, int n) { return (a + (1LL << (n - 1)) + (a >> 63)) >> n; }
@@ -87,8 +88,8 @@ __device__ __forceinline__ fxc fx_cmul(fxc z, int4 w) {
 __device__ __forceinline__ fx fx_rsqrt2(fx a) {
   constexpr int c1 = 1257966796, c0 = 102865788;
   const int a1 = fx_s1(a), a0 = fx_lo(a);
-  const fx m = (1LL << 31) + mw(a1, c0) + mw(a0, c1);
-  return a - ((fx)fx_hi(m) + mw(a1, c1));
+  const fx m = (1LL << 31) + mw(a1, -c0) + mw(a0, -c1);
+  return a + mw(a1, -c1) + (fx)fx_hi(m);
 }
 
 __device__ __forceinline__ void fx_dft4(fxc& a0, fxc& a1, fxc& a2, fxc& a3) {
@@ -128,7 +129,7 @@ template <int TOP>
 __device__ __forceinline__ fx fx_from(double v, int emax) {
   const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
   const unsigned m = (hi & 0xfffffu) | 0x100000u;
-  const int sh = emax - (int)((hi >> 20) & 0x7ff) + (63 - TOP);
+  const int sh = (int)(((unsigned)(emax + 63 - TOP) << 20) + 0xfffffu - (hi & 0x7fffffffu)) >> 20;
   unsigned long long u = ((unsigned long long)__funnelshift_l(lo, m, 11) << 32) | (lo << 11);
   asm("shr.u64 %0, %0, %1;" : "+l"(u) : "r"(sh));   // PTX clamps the amount: zeros and tiny values give 0
   const fx s = (fx)((int)hi >> 31);
@@ -142,9 +143,11 @@ __device__ __forceinline__ double fx_to(fx a, int sc20) {
   return __hiloint2double(hi ? hi + sc20 : 0, __double2loint(d));
 }
 
-__device__ __forceinline__ int fx_mag(fxc z) {   // OR of the components' magnitudes, high words
+// OR over components of x ^ 2x, high words: its top bit is one above the
+// largest magnitude's
+__device__ __forceinline__ int fx_mag(fxc z) {
   const int a = fx_hi(z.x), b = fx_hi(z.y);
-  return (a ^ (a >> 31)) | (b ^ (b >> 31));
+  return (a ^ (a + a)) | (b ^ (b + b));
 }
 
 // One value per line reduced over the line's threads.  Lines inside one warp
@@ -209,22 +212,26 @@ struct FxSmem {
   }
 };
 
-// Shift a line whose magnitudes' OR has high word m to top bit FX_TOP_TW; the exponent follows
-template <int E>
+// Shift a line whose fx_mag OR is m to top bit FX_TOP_TW, the exponent
+// following, unless it is near enough (normal data stays within the range by
+// itself: a radix-8 stage grows it by 1.5 bits, the product takes 2)
+template <int MAX, int E>
 __device__ __forceinline__ void fx_level(fxc (&v)[E], int m, int& sc) {
-  const int n = __clz(m) - (31 - (FX_TOP_TW - 32));
+  const int top = 62 - __clz(m);   // bit of the line's largest magnitude
+  if (top >= FX_TOP_MIN && top <= MAX) return;
+  const int n = FX_TOP_TW - top;
   sc -= n;
   if (n > 0) {
 #pragma unroll
     for (int e = 0; e < E; e++) v[e] = {v[e].x << n, v[e].y << n};
-  } else if (n < 0) {
+  } else {
 #pragma unroll
     for (int e = 0; e < E; e++) v[e] = {fx_sar(v[e].x, -n), fx_sar(v[e].y, -n)};
   }
 }
 
 // the Stockham stages of run_stages64, with the line's exponent carried along
-template <int LOGL, int C, bool COLS, bool WARP_ONLY, int S, class SM>
+template <int LOGL, int C, bool COLS, bool WARP_ONLY, bool PAIRS, int S, class SM>
 __device__ __forceinline__ void fx_stages(fxc (&v)[Sched64<LOGL>::E], int t, int c, const int4* tw, const SM& sm,
                                           int* slots, int& sc) {
   using Sc = Sched64<LOGL>;
@@ -267,8 +274,8 @@ __device__ __forceinline__ void fx_stages(fxc (&v)[Sched64<LOGL>::E], int t, int
       for (int e = 0; e < E; e++) v[e] = sm.get(c, t + T * e);
       if constexpr (!Ln::REG) mag = slots[(S + 1) * C + c];
       if constexpr (S + 1 < Sc::NSTAGES - 1) line_sync<WARP_ONLY>();   // every gather is done before the next scatter
-      fx_level(v, mag, sc);
-      fx_stages<LOGL, C, COLS, WARP_ONLY, S + 1>(v, t, c, tw, sm, slots, sc);
+      fx_level<PAIRS && S + 1 == Sc::NSTAGES - 1 ? FX_TOP_TW : FX_TOP_MAX>(v, mag, sc);
+      fx_stages<LOGL, C, COLS, WARP_ONLY, PAIRS, S + 1>(v, t, c, tw, sm, slots, sc);
     }
   }
 }
@@ -383,7 +390,7 @@ __device__ __forceinline__ void line_fx64_body(const LineParams& p, long long ct
     }
   }
 
-  fx_stages<LOGL, C, COLS, WARP_ONLY, 0>(v, t, c, tw, sm, slots, sc);
+  fx_stages<LOGL, C, COLS, WARP_ONLY, KIND == LK_R2C, 0>(v, t, c, tw, sm, slots, sc);
 
   if constexpr (KIND == LK_C2C && TSTORE) {
     if constexpr (Sc::NSTAGES > 1) __syncthreads();
