@@ -85,6 +85,17 @@ def test_strided(dims, dev):
     assert rel(run("c", dims, 1, (a, b), dev), sfft.fftn(z).reshape(1, -1)) <= TOL
 
 
+# lines of 8192 points in two passes, axes of 2^20 points in three
+@pytest.mark.parametrize("kind,dims,batch", [("c", [8192], 9), ("ci", [2, 8192], 5), ("c", [1 << 20], 8)])
+def test_split_lines(kind, dims, batch, dev):
+    rng = np.random.default_rng(5)
+    a, b = rng.standard_normal((2, batch, int(np.prod(dims))))
+    z = (a.astype(np.clongdouble) + 1j * b.astype(np.longdouble)).reshape([batch] + dims)[-2:]
+    axes = tuple(range(1, len(dims) + 1))
+    ref = sfft.fftn(z, axes=axes) if kind == "c" else sfft.ifftn(z, axes=axes, norm="forward")
+    assert rel(run(kind, dims, batch, (a, b), dev)[-2:], ref.reshape(2, -1)) <= TOL
+
+
 # spiky and smooth lines, and neighbours of other scales, up to the ends of the range
 @pytest.mark.parametrize("n", [8, 64, 256, 4096])
 def test_scales(n, dev):
