@@ -4,6 +4,7 @@
 // multi.hpp:343-414): thread (q, k), k in [0, L/2], owns the pair (k, L-k)
 // of line q, so the pass may run in place.
 #include "kernels64.h"
+#include "line_fx64.cuh"
 
 namespace agb {
 
@@ -27,58 +28,101 @@ __device__ __forceinline__ double ld64(const float* base, long long off) {
 
 }  // namespace
 
+// The pair (line q, bin k in [0, L/2]) of thread idx of a real pass.  64-bit
+// division only where the index needs it (the FP32 pass, bound by its loads,
+// gains nothing from this).
+__device__ __forceinline__ void real_pass_index(const RealPassParams& p, long long idx, long long* q, long long* k) {
+  const long long half = p.L / 2 + 1;
+  const long long n = p.lines_fastest ? p.nlines : half;
+  long long a, b;   // idx = a * n + b
+  if (p.nlines * half < 0xffff0000LL) {
+    const unsigned m = (unsigned)idx / (unsigned)n;
+    a = m;
+    b = (unsigned)idx - m * (unsigned)n;
+  } else {
+    a = idx / n;
+    b = idx - a * n;
+  }
+  *q = p.lines_fastest ? b : a;
+  *k = p.lines_fastest ? a : b;
+}
+
+// One pair of bins in block fixed point (line_fx64.cuh), its four values
+// sharing an exponent: FP64 instructions bound this pass on the FP64 pipe (32
+// x 2^19 complex points 437 us of a 2^20-point real forward's 951).  One
+// product serves both bins: bin L-k's a and b are the conjugates of bin k's
+// (2^20 x 32 r2c 952 -> 610 us, c2r 918 -> 618, 2^15 x 512 r2c 419 -> 248).
+// The values the fixed-point form leaves out take the FP64 form.
+template <bool INVERSE>
+__device__ __forceinline__ void pair64(double2 s0, double2 s1, const int4* rtw, long long k, long long L, double2* xk,
+                                       double2* xl) {
+  const int top = max(max(d_hi(s0.x) & 0x7fffffff, d_hi(s0.y) & 0x7fffffff),
+                      max(d_hi(s1.x) & 0x7fffffff, d_hi(s1.y) & 0x7fffffff));
+  const int emax = top >> 20;
+  if (emax < FX_EXP_MIN || emax > FX_EXP_MAX) {
+    *xk = INVERSE ? pre_one64(s0, s1, ldz(rtw + k)) : post_one64(s0, s1, ldz(rtw + k));
+    *xl = INVERSE ? pre_one64(s1, s0, ldz(rtw + (L - k))) : post_one64(s1, s0, ldz(rtw + (L - k)));
+    return;
+  }
+  constexpr int TOP = 59;   // components < 2^60: sums < 2^61, products < 2^62, results < 2^62.6
+  int4 w = __ldg(rtw + k);
+  const fxc u0 = {fx_from<TOP>(s0.x, emax), fx_from<TOP>(s0.y, emax)};
+  const fxc u1 = {fx_from<TOP>(s1.x, emax), fx_from<TOP>(s1.y, emax)};
+  const fxc a = {u0.x + u1.x, u0.y - u1.y};
+  fxc b;
+  int sc20;
+  if constexpr (INVERSE) {
+    w.z = -w.z;
+    w.w = -w.w;
+    b = fx_cmul<true>({u1.x - u0.x, -u1.y - u0.y}, w);
+    sc20 = (emax - 1023 - TOP) * (1 << 20);
+  } else {   // a and b are twice the pass's: the exponent has the 1/2
+    b = fx_cmul<true>({u0.x - u1.x, u0.y + u1.y}, w);
+    sc20 = (emax - 1023 - TOP - 1) * (1 << 20);
+  }
+  const fxc x = csub_i(a, b), y = cadd_i(a, b);   // a - i b; conj(a + i b)
+  *xk = make_double2(fx_to(x.x, sc20), fx_to(x.y, sc20));
+  *xl = make_double2(fx_to(y.x, sc20), fx_to(-y.y, sc20));
+}
+
 __global__ void real_pass_kernel64(const RealPassParams p) {
   pdl_enter();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long half = p.L / 2 + 1;
   long long q, k;
-  if (p.lines_fastest) {
-    q = idx % p.nlines;
-    k = idx / p.nlines;
-  } else {
-    k = idx % half;
-    q = idx / half;
-  }
+  real_pass_index(p, idx, &q, &k);
   if (q >= p.nlines || k >= half) return;
   const long long L = p.L;
   const int4* rtw = reinterpret_cast<const int4*>(p.rtw);
   const long long bi = line_off(p.in, q), bo = line_off(p.out, q);
   const long long ik = bi + k * p.in.es, iL = bi + (L - k) * p.in.es;
   const long long ok = bo + k * p.out.es, oL = bo + (L - k) * p.out.es;
-  const double2 s0 = make_double2(ld64(p.in.re, ik), ld64(p.in.im, ik));
-  const double2 s1 = make_double2(ld64(p.in.re, iL), ld64(p.in.im, iL));
   double* ore = reinterpret_cast<double*>(p.out.re);
   double* oim = reinterpret_cast<double*>(p.out.im);
-  if (!p.inverse) {
-    if (k == 0) {
+  if (k == 0) {
+    if (!p.inverse) {
+      const double2 s0 = make_double2(ld64(p.in.re, ik), ld64(p.in.im, ik));
       ore[ok] = s0.x + s0.y;
       oim[ok] = 0.0;
       ore[oL] = s0.x - s0.y;
       oim[oL] = 0.0;
-      return;
+    } else {
+      const double x0 = ld64(p.in.re, ik), xL = ld64(p.in.re, iL);
+      ore[ok] = x0 + xL;
+      oim[ok] = x0 - xL;
     }
-    const double2 xk = post_one64(s0, s1, ldz(rtw + k));
-    const double2 xl = post_one64(s1, s0, ldz(rtw + L - k));
-    ore[ok] = xk.x;
-    oim[ok] = xk.y;
-    if (L - k != k) {
-      ore[oL] = xl.x;
-      oim[oL] = xl.y;
-    }
-  } else {
-    if (k == 0) {
-      ore[ok] = s0.x + s1.x;
-      oim[ok] = s0.x - s1.x;
-      return;
-    }
-    const double2 zk = pre_one64(s0, s1, ldz(rtw + k));
-    const double2 zl = pre_one64(s1, s0, ldz(rtw + L - k));
-    ore[ok] = zk.x;
-    oim[ok] = zk.y;
-    if (L - k != k) {
-      ore[oL] = zl.x;
-      oim[oL] = zl.y;
-    }
+    return;
+  }
+  const double2 s0 = make_double2(ld64(p.in.re, ik), ld64(p.in.im, ik));
+  const double2 s1 = make_double2(ld64(p.in.re, iL), ld64(p.in.im, iL));
+  double2 xk, xl;
+  if (p.inverse) pair64<true>(s0, s1, rtw, k, L, &xk, &xl);
+  else pair64<false>(s0, s1, rtw, k, L, &xk, &xl);
+  ore[ok] = xk.x;
+  oim[ok] = xk.y;
+  if (L - k != k) {
+    ore[oL] = xl.x;
+    oim[oL] = xl.y;
   }
 }
 

@@ -132,3 +132,26 @@ def test_non_finite_lines_stay_their_own(n, dev):
     z = a.astype(np.clongdouble) + 1j * b.astype(np.longdouble)
     assert rel(got[good], sfft.fft(z[good])) <= TOL
     assert abs(float(got[23, 0].real) - n * 5e-320) <= 5e-324 * n
+
+
+# the standalone real pass (lines longer than one CTA): scales to the ends of
+# the range side by side, and a line that is not finite
+def test_long_real_lines(dev):
+    n = 1 << 15
+    rng = np.random.default_rng(1)
+    scale = np.array([1.0, 1e-300, 1e300, 1e-3, 0.0, 1e5])
+    a = rng.standard_normal((len(scale), n)) * scale[:, None]
+    a[3, 100] = np.nan
+    good = [0, 1, 2, 5]
+    s = np.exp2(-np.floor(np.log2(np.abs(a[good]).max(1))))[:, None]
+    ref = sfft.rfft(a[good].astype(np.longdouble))
+    got = run("r", [n], len(scale), (a,), dev)
+    assert rel(got[good] * s, ref * s) <= TOL
+    assert np.all(got[4] == 0) and not np.isfinite(got[3].astype(np.complex128)).any()
+    sr, si = ref.real.astype(np.float64), ref.imag.astype(np.float64)
+    si[:, [0, -1]] = np.nan
+    back = run("ri", [n], 4, (sr * 2.0 ** -20, si * 2.0 ** -20), dev)
+    z = sr.astype(np.clongdouble)
+    z.imag[:, 1:-1] = si[:, 1:-1]
+    want = sfft.irfft(z * s, n) * n
+    assert rel(back * s * 2.0 ** 20, want) <= TOL
