@@ -28,7 +28,10 @@ struct LineKernel {
   int threads;         // T * C
   size_t smem;         // bytes of dynamic shared memory
   int halves;          // CTAs per tile of C lines (2: the split R2C pass)
-  int stage_logl;      // log2 length of the stage twiddle table the kernel reads
+  int stage_logl;      // log2 length of the stage twiddle table the kernel reads (+ kWideTable: the
+                       // table of the 32-points-per-thread schedule)
+  int grouped_threads; // threads, shared memory of the grouped forms (16 points per thread at every length:
+  size_t grouped_smem; // their stage table is the one without kWideTable)
   LineKernelTmaFn tma; // the same pass with its input tile loaded by TMA (cols passes over
                        // split planes), or null
   GroupedKernelFn grouped_tma;   // its grouped form (queue segments with tensor maps), or null
@@ -46,6 +49,7 @@ struct LineKernel {
                                      // axis); logl is then log2 of the row length; 0 for line kernels
 };
 
+constexpr int kWideTable = 32;
 constexpr int ROWS_MAX_LOG = 14;   // rows mode: one CTA up to 16384 points
 constexpr int COLS_MAX_LOG = 11;   // cols mode: one CTA up to 2048 points
 
@@ -88,7 +92,8 @@ bool get_cols_tma(int logl, int kind, LineKernel* out);
 // 2^10 points with TMA-loaded input tiles (k_cols_tma_ts.cu)
 bool get_cols_tma_tstore(int logl, LineKernel* out);
 // complex cols passes over interleaved input pairs (pairs bit 0 set: 1 or
-// 3), plain or with the transposing store, 2^8 and 2^9 points, with TMA
+// 3), plain or with the transposing store, 2^8 to 2^10 points, and split input with output pairs
+// (pairs 2, not transposing, 2^9 and 2^10 points), with TMA
 // loads of the interleaved tile (k_cols_tma_pairs.cu)
 bool get_cols_tma_pairs(int logl, bool tstore, int pairs, LineKernel* out);
 
@@ -165,6 +170,7 @@ constexpr int lines_per_cta_k() {
 template <int LOGL, bool COLS, int KIND, bool TSTORE, bool TC = false, int UNIT = 0, int CC = 0>
 LineKernel make_line_kernel() {
   constexpr int C = CC ? CC : lines_per_cta_k<LOGL, COLS, KIND>();
+  using Sc = SchedOf<LOGL, COLS, KIND, TC>;
   static_assert(!TC || (size_t)LineSmem<LOGL, C, COLS, TSTORE, TC>::FLOAT2S * 8 >= (size_t)(Sched<LOGL>::T * C / 128) * 16384,
                 "TC operand tiles must fit in the exchange buffer");
   LineKernel k;
@@ -179,11 +185,13 @@ LineKernel make_line_kernel() {
   k.cols = COLS;
   k.kind = KIND == LK_R2C_HALF ? LK_R2C : KIND;
   k.halves = KIND == LK_R2C_HALF ? 2 : 1;
-  k.stage_logl = LOGL;
+  k.stage_logl = LOGL + (Sc::E == 32 ? kWideTable : 0);
   k.tstore = TSTORE;
   k.lines_per_cta = C;
-  k.threads = Sched<LOGL>::T * C;
-  k.smem = (size_t)LineSmem<LOGL, C, COLS, TSTORE, TC>::FLOAT2S * sizeof(float2);
+  k.threads = Sc::T * C;
+  k.smem = (size_t)SmemOf<LOGL, C, COLS, KIND, TSTORE, TC>::FLOAT2S * sizeof(float2);
+  k.grouped_threads = Sched<LOGL>::T * C;
+  k.grouped_smem = (size_t)LineSmem<LOGL, C, COLS, TSTORE, TC>::FLOAT2S * sizeof(float2);
   return k;
 }
 
@@ -191,7 +199,7 @@ LineKernel make_line_kernel() {
 template <int LOGL, int KIND, int CC = 0, bool TSTORE = false, int UNIT = 0>
 LineKernel make_tma_kernel() {
   constexpr int C = CC ? CC : lines_per_cta_k<LOGL, true, KIND>();
-  static_assert((size_t)LineSmem<LOGL, C, true, TSTORE, false>::FLOAT2S * sizeof(float2) >=
+  static_assert((size_t)SmemOf<LOGL, C, true, KIND, TSTORE>::FLOAT2S * sizeof(float2) >=
                     (size_t)2 * (1 << LOGL) * C * sizeof(float),
                 "the input tile fits the exchange buffer it aliases");
   static_assert(C * sizeof(float) % 16 == 0, "tile columns span whole 16-byte units");
@@ -235,8 +243,8 @@ LineKernel make_plane_kernel() {
   k.tc = 0;
   k.unit = UNIT;
   k.lines_per_cta = PS::PPC * PS::D1;   // rows per CTA: PPC planes of D1 rows
-  k.threads = PS::NT;
-  k.smem = (size_t)PS::FLOAT2S * sizeof(float2);
+  k.threads = k.grouped_threads = PS::NT;
+  k.smem = k.grouped_smem = (size_t)PS::FLOAT2S * sizeof(float2);
   k.halves = 1;
   k.stage_logl = LOG2;
   return k;
@@ -252,7 +260,9 @@ LineKernel make_pipe_kernel() {
   k.grouped_pipe = TSTORE ? nullptr : &line_fft_pipe_grouped<LOGL, C, KIND>;
   static_assert(LOGL == 11 || LOGL == 10, "the pipelined kernels are built for 1024- and 2048-point lines");
   k.pipe_smem = ((size_t)2 * (1 << LOGL) + pipe_rows<LOGL>()) * C * sizeof(float);   // raw tile + exchange rows
-  k.pipe_ctas = 1024 / (Sched<LOGL>::T * C);
+  k.pipe_ctas = pipe_ctas<LOGL, C>();
+  static_assert(std::is_same_v<PipeSched<LOGL>, SchedOf<LOGL, true, KIND>>,
+                "the one-tile and the pipelined form share block size and stage table");
   return k;
 }
 

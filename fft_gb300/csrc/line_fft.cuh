@@ -331,6 +331,31 @@ __device__ __forceinline__ double ldin(const double* p) {
   return v;
 }
 
+}  // namespace agb
+#include "line_wide.cuh"
+namespace agb {
+
+// Which kernels take the 32-points-per-thread schedule of line_wide.cuh:
+// complex and plain real cols passes of 512 and 1024 points (and the split
+// 2048-point R2C pass).  Measured against 16 points per thread, us: 2^20 c2c
+// x 16 127 -> 115, x 64 450 -> 420, 1024^2 x 64 368 -> 365, 512^2 x 37 58.7 ->
+// 57.0 (as pairs 63.5 -> 60.2), 2^20 r2c x 64 300 -> 286, c2r 334 -> 297,
+// 2048^2 c2r x 16 211 -> 192, r2c x 4 65.0 -> 62.2, 4096^2 r2c 74.4 -> 72.8.
+// The paired real passes are slower that way (2^20 r2c x 64 286 vs 318), and
+// so are the queue's grouped kernels (GROUPED), which share the SMs with
+// other groups (1000 mixed transforms 1005 vs 1040).
+template <int LOGL, bool COLS, int KIND, bool TC, bool GROUPED>
+constexpr bool is_wide() {
+  return COLS && !TC && !GROUPED && (LOGL == 9 || LOGL == 10) && KIND <= LK_R2C_HALF;
+}
+template <int LOGL, bool COLS, int KIND, bool TC = false, bool GROUPED = false>
+using SchedOf =
+    std::conditional_t<is_wide<LOGL, COLS, KIND, TC, GROUPED>(), Wide<LOGL == 9 ? 9 : 10>, Sched<LOGL>>;
+template <int LOGL, int C, bool COLS, int KIND, bool TSTORE, bool TC = false, bool GROUPED = false>
+using SmemOf = std::conditional_t<is_wide<LOGL, COLS, KIND, TC, GROUPED>(),
+                                  WideSmem<LOGL == 9 ? 9 : 10, C == 16 ? 16 : 8, TSTORE>,
+                                  LineSmem<LOGL, C, COLS, TSTORE, TC>>;
+
 // One Stockham stage: B = E/R butterflies per thread, butterfly b = t + T*u
 // reads slots u + B*r, applies W_{NS*R}^{r*(b mod NS)}, DFT-R, and either
 // scatters to shared memory (non-last) or keeps the canonical layout (last).
@@ -428,6 +453,22 @@ constexpr int min_ctas() {
   return AFFT_REG_CAP ? (65536 / (AFFT_REG_CAP * NT) > 0 ? 65536 / (AFFT_REG_CAP * NT) : 1) : 1;
 }
 
+// CTAs per SM of a kernel: the threads of the wide schedule hold 128
+// registers, 512 of them to an SM
+template <class Sc, int C>
+constexpr int cta_bound() {
+  return Sc::E == 32 ? 512 / (Sc::T * C) : min_ctas<Sc::T * C>();
+}
+
+// All stages of a kernel's schedule
+template <int LOGL, int C, bool COLS, int KIND, bool TSTORE, bool WARP_ONLY, bool TC, bool GROUPED, class SM, int E>
+__device__ __forceinline__ void line_stages(float2 (&v)[E], int t, int c, const float2* tw, const SM& sm,
+                                            TcState* ts = nullptr) {
+  if constexpr (is_wide<LOGL, COLS, KIND, TC, GROUPED>()) wide_stages<LOGL, true>(v, t, c, tw, sm);
+  else if constexpr (KIND == LK_R2C_HALF) run_stages<LOGL, C, COLS, WARP_ONLY, 0>(v, t, c, tw, sm);
+  else run_stages<LOGL, C, COLS, WARP_ONLY, 0, TC, packed_bfly<LOGL, COLS, TSTORE>()>(v, t, c, tw, sm, ts);
+}
+
 // The real forward (R2C) pass along a strided axis of Z = 2 Lh complex
 // points (Lh = 2^LOGL), split over two CTAs per tile of C lines.  With the
 // first radix-2 step of a decimation in frequency,
@@ -440,13 +481,13 @@ constexpr int min_ctas() {
 // m with Lh - 1 - m.  Both CTAs of a tile read the whole tile (the second
 // read is served by L2).  rtw = W_{4Lh}^k, k < 2 Lh, as for the unsplit pass;
 // W_{2Lh}^j = rtw[2j].  The stage twiddles are those of Lh.
-template <int LOGL, int C>
+template <int LOGL, int C, bool GROUPED>
 __device__ __forceinline__ void r2c_half_body(const LineParams& p, long long cta) {
-  using Sc = Sched<LOGL>;
+  using Sc = SchedOf<LOGL, true, LK_R2C_HALF, false, GROUPED>;
   constexpr int Lh = Sc::L, E = Sc::E, T = Sc::T, L = 2 * Lh;
   constexpr bool WARP_ONLY = T * C <= 32;
   extern __shared__ __align__(1024) float2 smem_raw[];
-  LineSmem<LOGL, C, true, false, false> sm{smem_raw};
+  SmemOf<LOGL, C, true, LK_R2C_HALF, false, false, GROUPED> sm{smem_raw};
   const int tid = threadIdx.x;
   const int c = tid % C, t = tid / C;
   const int h = (int)(cta & 1);
@@ -472,7 +513,7 @@ __device__ __forceinline__ void r2c_half_body(const LineParams& p, long long cta
     for (int e = 0; e < E; e++) v[e] = make_float2(0.f, 0.f);
   }
 
-  run_stages<LOGL, C, true, WARP_ONLY, 0>(v, t, c, p.tw, sm);
+  line_stages<LOGL, C, true, LK_R2C_HALF, false, WARP_ONLY, false, GROUPED>(v, t, c, p.tw, sm);
 
   // real forward post-pass on this half's bins (the formula of the unsplit
   // pass below: X[k] = a - i b, X[0] and X[L] from Z[0])
@@ -971,7 +1012,7 @@ __device__ __forceinline__ void bulk_stage_out(const float2 (&v)[E], int t, int 
 // planes in the tile's buffer (bulk_stage_out) for the caller to store by TMA
 // (line_fft_tma_bulk) instead of storing them itself.
 template <int LOGL, int C, bool COLS, int KIND, bool TSTORE, bool TC = false, int UNIT = 0, bool TMA = false,
-          bool BULK = false>
+          bool BULK = false, bool GROUPED = false>
 __device__ __forceinline__ void line_fft_body(const LineParams& p, long long cta, TcState* ts = nullptr) {
   static_assert(!TMA || (COLS && !TC && (UNIT == 0 || KIND == LK_C2C) && (!TSTORE || KIND == LK_C2C)),
                 "TMA tiles: cols passes");
@@ -979,7 +1020,7 @@ __device__ __forceinline__ void line_fft_body(const LineParams& p, long long cta
                 "TMA stores: split C2C and C2R cols tiles");
   if constexpr (KIND == LK_R2C_HALF) {
     static_assert(COLS && !TSTORE && !TC, "the split R2C pass is a plain cols pass");
-    r2c_half_body<LOGL, C>(p, cta);
+    r2c_half_body<LOGL, C, GROUPED>(p, cta);
     return;
   }
   if constexpr (KIND == LK_R2C_PAIRED) {
@@ -992,14 +1033,14 @@ __device__ __forceinline__ void line_fft_body(const LineParams& p, long long cta
     c2r_paired_body<LOGL, C, (UNIT & 2) != 0>(p, cta);
     return;
   }
-  using Sc = Sched<LOGL>;
+  using Sc = SchedOf<LOGL, COLS, KIND, TC, GROUPED>;
   constexpr int L = Sc::L, E = Sc::E, T = Sc::T;
   constexpr int RU = COLS ? 0 : UNIT;       // rows: unit-stride variants
   constexpr int CPAIRS = COLS ? UNIT : 0;   // cols: interleaved-pair input / output
   // a line lives inside one warp: rows mode with T <= 32, or a single line
   constexpr bool WARP_ONLY = (!COLS && T <= 32) || (T * C <= 32);
   extern __shared__ __align__(1024) float2 smem_raw[];
-  LineSmem<LOGL, C, COLS, TSTORE, TC> sm{smem_raw};
+  SmemOf<LOGL, C, COLS, KIND, TSTORE, TC, GROUPED> sm{smem_raw};
 
   const int tid = threadIdx.x;
   const int c = COLS ? (tid % C) : (tid / T);
@@ -1171,7 +1212,7 @@ __device__ __forceinline__ void line_fft_body(const LineParams& p, long long cta
     }
   }
 
-  run_stages<LOGL, C, COLS, WARP_ONLY, 0, TC, packed_bfly<LOGL, COLS, TSTORE>()>(v, t, c, p.tw, sm, ts);
+  line_stages<LOGL, C, COLS, KIND, TSTORE, WARP_ONLY, TC, GROUPED>(v, t, c, p.tw, sm, ts);
 
   if constexpr (KIND == LK_C2C) {
     if constexpr (TSTORE) {
@@ -1188,18 +1229,18 @@ __device__ __forceinline__ void line_fft_body(const LineParams& p, long long cta
         const long long base = line_off(p.out, q2);
         const bool inv = p.inverse;
         // one branch-free loop per case, so the twiddle loads issue together
-        // tw: 0 none, 1 matrix table, 2 hi/lo pair
+        // (every transposing pass has the twiddle; the hi/lo pair is the
+        // no-allocation entry point's, which launches the split LSU kernels)
+        constexpr bool HILO = !TMA && UNIT == 0;
         // the four-step passes store with unit element stride: compile-time
         // offsets from one pointer per array; other strides as the loads
         const long long S = (long long)T * p.out.es;
         float* pr = p.out.re + base + (long long)t2 * p.out.es;
         float* pi = p.out.im + base + (long long)t2 * p.out.es;
-        auto emit = [&](auto tw, auto unit) {
-          constexpr int TW = decltype(tw)::value;
+        auto emit = [&](auto full, auto unit) {
 #pragma unroll
           for (int e = 0; e < E; e++) {
-            float2 x = sm.get(c2, t2 + T * e);
-            if constexpr (TW) x = cmul(x, fourstep_twiddle<L, TW == 1>(p, q2, t2 + T * e));
+            float2 x = cmul(sm.get(c2, t2 + T * e), fourstep_twiddle<L, decltype(full)::value>(p, q2, t2 + T * e));
             x = inv ? cswap(x) : x;
             const long long o = decltype(unit)::value ? (long long)(T * e) : e * S;
             pr[o] = x.x;
@@ -1207,9 +1248,8 @@ __device__ __forceinline__ void line_fft_body(const LineParams& p, long long cta
           }
         };
         auto emit_tw = [&](auto unit) {
-          if (!p.tw_n) emit(std::integral_constant<int, 0>{}, unit);
-          else if (p.tw_full) emit(std::integral_constant<int, 1>{}, unit);
-          else emit(std::integral_constant<int, 2>{}, unit);
+          if (!HILO || p.tw_full) emit(std::true_type{}, unit);
+          else if constexpr (HILO) emit(std::false_type{}, unit);
         };
         bool stored = false;
         if constexpr ((CPAIRS & 2) != 0) {
@@ -1218,18 +1258,11 @@ __device__ __forceinline__ void line_fft_body(const LineParams& p, long long cta
           float* pz = p.out.re + base + 2LL * t2;
           if (p.out.es == 2 && !(reinterpret_cast<uintptr_t>(pz) & 7)) {
             float2* pp = reinterpret_cast<float2*>(pz);
-            auto emit2 = [&](auto tw) {
-              constexpr int TW = decltype(tw)::value;
 #pragma unroll
-              for (int e = 0; e < E; e++) {
-                float2 x = sm.get(c2, t2 + T * e);
-                if constexpr (TW) x = cmul(x, fourstep_twiddle<L, TW == 1>(p, q2, t2 + T * e));
-                pp[T * e] = inv ? cswap(x) : x;
-              }
-            };
-            if (!p.tw_n) emit2(std::integral_constant<int, 0>{});
-            else if (p.tw_full) emit2(std::integral_constant<int, 1>{});
-            else emit2(std::integral_constant<int, 2>{});
+            for (int e = 0; e < E; e++) {
+              const float2 x = cmul(sm.get(c2, t2 + T * e), fourstep_twiddle<L, true>(p, q2, t2 + T * e));
+              pp[T * e] = inv ? cswap(x) : x;
+            }
             stored = true;
           }
         }
@@ -1243,10 +1276,11 @@ __device__ __forceinline__ void line_fft_body(const LineParams& p, long long cta
     } else {
       // four-step twiddles only occur in cols passes
       if constexpr (COLS) {
-        if (p.tw_n && p.tw_full) {
+        constexpr bool HILO = !TMA && UNIT == 0;   // as above
+        if (p.tw_n && (!HILO || p.tw_full)) {
 #pragma unroll
           for (int e = 0; e < E; e++) v[e] = cmul(v[e], fourstep_twiddle<L, true>(p, q, t + T * e));
-        } else if (p.tw_n) {
+        } else if (HILO && p.tw_n) {
 #pragma unroll
           for (int e = 0; e < E; e++) v[e] = cmul(v[e], fourstep_twiddle<L, false>(p, q, t + T * e));
         }
@@ -1475,7 +1509,7 @@ __device__ __forceinline__ void tc_teardown(const TcState& S) {
 }
 
 template <int LOGL, int C, bool COLS, int KIND, bool TSTORE, bool TC = false, int UNIT = 0>
-__global__ void __launch_bounds__(Sched<LOGL>::T * C, min_ctas<Sched<LOGL>::T * C>())
+__global__ void __launch_bounds__(SchedOf<LOGL, COLS, KIND, TC>::T * C, cta_bound<SchedOf<LOGL, COLS, KIND, TC>, C>())
 line_fft(const LineParams p) {
   pdl_enter();
   if constexpr (TC) {
@@ -1583,7 +1617,7 @@ __device__ __forceinline__ bool tma_load_tile(const LineParams& p, const TmaTile
 }
 
 template <int LOGL, int C, int KIND, bool TSTORE = false, int UNIT = 0>
-__global__ void __launch_bounds__(Sched<LOGL>::T * C, min_ctas<Sched<LOGL>::T * C>())
+__global__ void __launch_bounds__(SchedOf<LOGL, true, KIND>::T * C, cta_bound<SchedOf<LOGL, true, KIND>, C>())
 line_fft_tma(const LineParams p, const __grid_constant__ TmaTile tm) {
   __shared__ __align__(8) uint64_t mbar;
   extern __shared__ __align__(1024) float2 smem_raw[];
@@ -1680,7 +1714,7 @@ line_fft_grouped(const Segment* __restrict__ segs, const int* __restrict__ seg_o
       stage_params(sp, segs[sg].p);
       __syncthreads();   // parameters staged, the barrier's set-up visible
       if (!tma_wait_tile(mb, sp.err)) return;
-      line_fft_body<LOGL, C, true, KIND, TSTORE, false, UNIT, true>(sp, cta);
+      line_fft_body<LOGL, C, true, KIND, TSTORE, false, UNIT, true, false, true>(sp, cta);
     }
     return;
   }
@@ -1696,7 +1730,7 @@ line_fft_grouped(const Segment* __restrict__ segs, const int* __restrict__ seg_o
       __syncthreads();
       stage_params(sp, segs[sg].p);
       __syncthreads();
-      line_fft_body<LOGL, C, COLS, KIND, TSTORE, true, UNIT>(sp, v - segs[sg].cta0, &S);
+      line_fft_body<LOGL, C, COLS, KIND, TSTORE, true, UNIT, false, false, true>(sp, v - segs[sg].cta0, &S);
     }
     tc_teardown<Sched<LOGL>::T * C>(S);
   } else {
@@ -1705,7 +1739,7 @@ line_fft_grouped(const Segment* __restrict__ segs, const int* __restrict__ seg_o
       __syncthreads();   // a previous iteration is done with sp and the staging buffers
       stage_params(sp, segs[sg].p);
       __syncthreads();
-      line_fft_body<LOGL, C, COLS, KIND, TSTORE, false, UNIT>(sp, v - segs[sg].cta0);
+      line_fft_body<LOGL, C, COLS, KIND, TSTORE, false, UNIT, false, false, true>(sp, v - segs[sg].cta0);
     }
   }
 }

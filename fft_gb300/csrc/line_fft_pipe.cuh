@@ -15,7 +15,8 @@
 // 128 KB at 2048 points, as tma_load_tile lays it out) and a separate exchange buffer through
 // which the stages pass the re parts first, then the im parts.  Element j of
 // line c sits at float (j + j/8) * C + c there (one pad row per 8: 72 KB;
-// 1024-point tiles pad one row per 4, below).  A
+// 1024-point tiles run 32 points per thread, line_wide.cuh, and pad one row
+// per 32, below).  A
 // warp covers 4 consecutive threads t (lanes 8 apart share a line), so each
 // access touches 4 rows, and the padding puts them on 4 different 8-bank
 // groups for the radix-8 scatter (rows 8 apart), the radix-16 scatter
@@ -53,7 +54,7 @@
 #define AFFT_PIPE_C 8
 #endif
 // the 1024-point complex and C2R cols passes in this form too (8-line tiles,
-// two 512-thread CTAs per SM, 104 KB each)
+// two 256-thread CTAs per SM, 98 KB each)
 #ifndef AFFT_PIPE10
 #define AFFT_PIPE10 1
 #endif
@@ -111,39 +112,42 @@ constexpr bool pipe_bulk() {
                                   (KIND == LK_C2R && LOGL == 10 && AFFT_PIPE_BULK_C2R10));
 }
 
-// Rows of the exchange buffer.  2048-point schedule (radix 8, 16, 16; T =
-// 128): row = j + j/8.  Stage 0 scatters output e = u + 2 r of butterfly
-// b = t + 128 u to element 8 b + r, stage 1 output e of butterfly t to
-// element 128 (t / 8) + t % 8 + 8 e, and the gather takes element t + 128 e.
-// 1024-point schedule (radix 4, 16, 16; T = 64): row = j + j/4.  Stage 0
-// scatters output e = u + 4 r of butterfly b = t + 64 u to element 4 b + r,
-// stage 1 output e of butterfly t to element 64 (t / 4) + t % 4 + 4 e, the
-// gather takes element t + 64 e.  Each is base(t) + offset(e).
+// The pipelined kernels' schedules: 2048 points radix 8, 16, 16 with 16 points
+// per thread, 1024 points 32, 32 with 32 (line_wide.cuh).
+template <int LOGL>
+using PipeSched = std::conditional_t<LOGL == 10, Wide<10>, Sched<LOGL>>;
+
+// Rows of the exchange buffer.  2048 points (T = 128): row = j + j/8.  Stage 0
+// scatters output e = u + 2 r of butterfly b = t + 128 u to element 8 b + r,
+// stage 1 output e of butterfly t to element 128 (t / 8) + t % 8 + 8 e, and
+// the gather takes element t + 128 e.  1024 points (T = 32): row = j + j/32.
+// Stage 0 scatters output e of butterfly t to element 32 t + e, the gather
+// takes element t + 32 e.  Each is base(t) + offset(e).
 template <int LOGL>
 __host__ __device__ constexpr int pipe_rows() {
-  return LOGL == 11 ? 2048 + 2048 / 8 : 1024 + 1024 / 4;
+  return LOGL == 11 ? 2048 + 2048 / 8 : 1024 + 1024 / 32;
 }
 template <int LOGL>
 __device__ __forceinline__ int pipe_row(int j) {
-  return LOGL == 11 ? j + (j >> 3) : j + (j >> 2);
+  return LOGL == 11 ? j + (j >> 3) : j + (j >> 5);
 }
 template <int LOGL, int S>
 __device__ __forceinline__ int pipe_wbase(int t) {
   if constexpr (LOGL == 11) return S == 0 ? 9 * t : 144 * (t >> 3) + (t & 7);
-  else return S == 0 ? 5 * t : 80 * (t >> 2) + (t & 3);
+  else return 33 * t;
 }
 template <int LOGL, int S>
 __host__ __device__ constexpr int pipe_woff(int e) {
   if constexpr (LOGL == 11) return S == 0 ? 1152 * (e % 2) + e / 2 : 9 * e;
-  else return S == 0 ? 320 * (e % 4) + e / 4 : 5 * e;
+  else return e;
 }
 template <int LOGL>
 __device__ __forceinline__ int pipe_gbase(int t) {
-  return LOGL == 11 ? t + (t >> 3) : t + (t >> 2);
+  return LOGL == 11 ? t + (t >> 3) : t;
 }
 template <int LOGL>
 __host__ __device__ constexpr int pipe_goff(int e) {
-  return LOGL == 11 ? 144 * e : 80 * e;
+  return LOGL == 11 ? 144 * e : 33 * e;
 }
 
 // The transposing store's staging of 8-line 1024-point tiles: element k of
@@ -157,8 +161,8 @@ __device__ __forceinline__ int pipe_tsidx(int k, int c) { return k * 8 + ((c + (
 // TRAIL: the buffer is written again before the next CTA-wide barrier.
 // hook: run by every thread after the first barrier (the late tile issue).
 template <int LOGL, int C, int S, bool TRAIL, class Hook>
-__device__ __forceinline__ void pipe_exchange(float2 (&v)[Sched<LOGL>::E], int t, int c, float* xs, const Hook& hook) {
-  constexpr int E = Sched<LOGL>::E;
+__device__ __forceinline__ void pipe_exchange(float2 (&v)[PipeSched<LOGL>::E], int t, int c, float* xs, const Hook& hook) {
+  constexpr int E = PipeSched<LOGL>::E;
   float* w = xs + pipe_wbase<LOGL, S>(t) * C + c;
   const float* g = xs + pipe_gbase<LOGL>(t) * C + c;
   float nx[E];
@@ -182,10 +186,14 @@ __device__ __forceinline__ void pipe_exchange(float2 (&v)[Sched<LOGL>::E], int t
 // XOUT: the exchange buffer is written again after the stages (TMA stores,
 // the transposing store), so the last exchange ends with a barrier.
 template <int LOGL, int C, int KIND, bool XOUT, int S, class Hook>
-__device__ __forceinline__ void pipe_stages(float2 (&v)[Sched<LOGL>::E], int t, int c, const float2* tw,
+__device__ __forceinline__ void pipe_stages(float2 (&v)[PipeSched<LOGL>::E], int t, int c, const float2* tw,
                                             float* xs, const Hook& hook) {
-  using Sc = Sched<LOGL>;
-  if constexpr (S < Sc::NSTAGES) {
+  using Sc = PipeSched<LOGL>;
+  if constexpr (LOGL == 10) {
+    wide_stage1<LOGL, true>(v);
+    pipe_exchange<LOGL, C, 0, KIND == LK_R2C || XOUT>(v, t, c, xs, hook);
+    wide_stage2<LOGL, true>(v, t, tw);
+  } else if constexpr (S < Sc::NSTAGES) {
     constexpr int R = Sc::radix(S), NS = Sc::ns(S);
     // the butterflies with their outputs kept in registers (stage()'s last-stage form)
     stage<R, NS, Sc::E, Sc::T, true, false, 0, packed_bfly<LOGL, true>()>(v, t, c, tw + Sc::twoff(S), xs, false,
@@ -237,6 +245,12 @@ __device__ __forceinline__ void pipe_store_plane(const LineParams& p, const CUte
   asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }
 
+// CTAs per SM (64 registers a thread at 2048 points, 128 at 1024)
+template <int LOGL, int C>
+constexpr int pipe_ctas() {
+  return (LOGL == 10 ? 512 : 1024) / (PipeSched<LOGL>::T * C);
+}
+
 // The tile loop of the pipelined kernels.  This CTA takes tiles first,
 // first + gridDim.x, ... < ntiles; prep(v, &cta) returns the parameters of
 // tile v (and its CTA index within them), and issue(v) (thread 0) issues
@@ -251,11 +265,10 @@ __device__ __forceinline__ void pipe_store_plane(const LineParams& p, const CUte
 template <int LOGL, int C, int KIND, bool BULK, bool TSTORE, class Prep, class Issue>
 __device__ __forceinline__ void pipe_loop(long long first, long long ntiles, uint32_t mb, float* raw, float* xs,
                                           const TmaTile* tmo, const Prep& prep, const Issue& issue) {
-  using Sc = Sched<LOGL>;
+  using Sc = PipeSched<LOGL>;
   constexpr int L = Sc::L, E = Sc::E, T = Sc::T;
   static_assert(KIND == LK_C2C || KIND == LK_R2C || KIND == LK_C2R, "plain cols kinds");
-  static_assert(((LOGL == 11 && (C == 8 || C == 4) && Sc::radix(0) == 8) || (LOGL == 10 && C == 8 && Sc::radix(0) == 4)) &&
-                    E == 16,
+  static_assert((LOGL == 11 && (C == 8 || C == 4) && E == 16) || (LOGL == 10 && C == 8 && E == 32),
                 "the exchange rows are those of 8- or 4-line 2048-point and 8-line 1024-point tiles");
   static_assert(!BULK || KIND == LK_C2C || KIND == LK_C2R, "TMA stores: the complex and C2R passes");
   static_assert(!TSTORE || (KIND == LK_C2C && LOGL == 10 && C == 8 && !BULK),
@@ -363,13 +376,8 @@ __device__ __forceinline__ void pipe_loop(long long first, long long ntiles, uin
       __syncthreads();
 #pragma unroll
       for (int e = 0; e < E; e++) v[e] = make_float2(rx[e], xs[pipe_tsidx(t2 + T * e, c2)]);
-      if (p.tw_n && p.tw_full) {
 #pragma unroll
-        for (int e = 0; e < E; e++) v[e] = cmul(v[e], fourstep_twiddle<L, true>(p, q2, t2 + T * e));
-      } else if (p.tw_n) {
-#pragma unroll
-        for (int e = 0; e < E; e++) v[e] = cmul(v[e], fourstep_twiddle<L, false>(p, q2, t2 + T * e));
-      }
+      for (int e = 0; e < E; e++) v[e] = cmul(v[e], fourstep_twiddle<L, true>(p, q2, t2 + T * e));
       if (p.inverse) {
 #pragma unroll
         for (int e = 0; e < E; e++) v[e] = cswap(v[e]);
@@ -386,12 +394,9 @@ __device__ __forceinline__ void pipe_loop(long long first, long long ntiles, uin
       continue;   // the next tile's first write to the buffer follows its own barriers
     }
     if constexpr (KIND == LK_C2C) {
-      if (p.tw_n && p.tw_full) {
+      if (p.tw_n) {
 #pragma unroll
         for (int e = 0; e < E; e++) v[e] = cmul(v[e], fourstep_twiddle<L, true>(p, q, t + T * e));
-      } else if (p.tw_n) {
-#pragma unroll
-        for (int e = 0; e < E; e++) v[e] = cmul(v[e], fourstep_twiddle<L, false>(p, q, t + T * e));
       }
       if (p.inverse) {
 #pragma unroll
@@ -470,7 +475,7 @@ __device__ __forceinline__ void pipe_loop(long long first, long long ntiles, uin
 // One plan launch: tiles 0 .. ntiles - 1 of the parameters p, their input
 // maps tm (and output maps tmo for the TMA stores).
 template <int LOGL, int C, int KIND, bool TSTORE = false>
-__global__ void __launch_bounds__(Sched<LOGL>::T * C, 1024 / (Sched<LOGL>::T * C))
+__global__ void __launch_bounds__(PipeSched<LOGL>::T * C, pipe_ctas<LOGL, C>())
 line_fft_pipe(const __grid_constant__ LineParams p, const __grid_constant__ TmaTile tm,
               const __grid_constant__ TmaTile tmo, long long ntiles) {
   __shared__ __align__(8) uint64_t mbar;
@@ -479,12 +484,12 @@ line_fft_pipe(const __grid_constant__ LineParams p, const __grid_constant__ TmaT
   const uint32_t mb = smem_u32(&mbar), raw_s = smem_u32(raw);
   pdl_enter();
   pipe_loop<LOGL, C, KIND, pipe_bulk<LOGL, KIND>() && !TSTORE, TSTORE>(
-      blockIdx.x, ntiles, mb, raw, raw + 2 * Sched<LOGL>::L * C, &tmo,
+      blockIdx.x, ntiles, mb, raw, raw + 2 * PipeSched<LOGL>::L * C, &tmo,
       [&](long long tile, long long* cta) -> const LineParams& {
         *cta = tile;
         return p;
       },
-      [&](long long tile) { pipe_issue<Sched<LOGL>::L, C>(p.in.qmask, p.in.qshift, tm, tile, raw_s, mb); });
+      [&](long long tile) { pipe_issue<PipeSched<LOGL>::L, C>(p.in.qmask, p.in.qshift, tm, tile, raw_s, mb); });
 }
 
 // The queue form: the group's virtual tiles (segments of several transforms,
@@ -492,7 +497,7 @@ line_fft_pipe(const __grid_constant__ LineParams p, const __grid_constant__ TmaT
 // tile's loads go out from its segment's column mask, shift and maps, and
 // its parameters are staged in shared memory when its turn comes.
 template <int LOGL, int C, int KIND>
-__global__ void __launch_bounds__(Sched<LOGL>::T * C, 1024 / (Sched<LOGL>::T * C))
+__global__ void __launch_bounds__(PipeSched<LOGL>::T * C, pipe_ctas<LOGL, C>())
 line_fft_pipe_grouped(const Segment* __restrict__ segs, const int* __restrict__ seg_of, long long total) {
   __shared__ LineParams sp;
   __shared__ __align__(8) uint64_t mbar;
@@ -500,7 +505,7 @@ line_fft_pipe_grouped(const Segment* __restrict__ segs, const int* __restrict__ 
   float* raw = reinterpret_cast<float*>(smem_raw);
   const uint32_t mb = smem_u32(&mbar), raw_s = smem_u32(raw);
   pipe_loop<LOGL, C, KIND, false, false>(
-      blockIdx.x, total, mb, raw, raw + 2 * Sched<LOGL>::L * C, nullptr,
+      blockIdx.x, total, mb, raw, raw + 2 * PipeSched<LOGL>::L * C, nullptr,
       [&](long long v, long long* cta) -> const LineParams& {
         const int sg = __ldg(seg_of + v);
         *cta = v - __ldg(&segs[sg].cta0);
@@ -510,7 +515,7 @@ line_fft_pipe_grouped(const Segment* __restrict__ segs, const int* __restrict__ 
       },
       [&](long long v) {
         const int sg = __ldg(seg_of + v);
-        pipe_issue<Sched<LOGL>::L, C>(__ldg(&segs[sg].p.in.qmask), __ldg(&segs[sg].p.in.qshift), *segs[sg].tma,
+        pipe_issue<PipeSched<LOGL>::L, C>(__ldg(&segs[sg].p.in.qmask), __ldg(&segs[sg].p.in.qshift), *segs[sg].tma,
                                       v - __ldg(&segs[sg].cta0), raw_s, mb);
       });
 }
@@ -520,7 +525,7 @@ line_fft_pipe_grouped(const Segment* __restrict__ segs, const int* __restrict__ 
 // host's tma_tile rules for the output).  Thread 0 waits until the stores
 // have read the buffer before the CTA ends.
 template <int LOGL, int C, int KIND>
-__global__ void __launch_bounds__(Sched<LOGL>::T * C, min_ctas<Sched<LOGL>::T * C>())
+__global__ void __launch_bounds__(SchedOf<LOGL, true, KIND>::T * C, cta_bound<SchedOf<LOGL, true, KIND>, C>())
 line_fft_tma_bulk(const __grid_constant__ LineParams p, const __grid_constant__ TmaTile tm,
                   const __grid_constant__ TmaTile tmo) {
   constexpr int L = Sched<LOGL>::L;

@@ -1,0 +1,124 @@
+// Cols passes of 512 and 1024 points with 32 points per thread and two stages
+// (16 or 32, then 32 points) instead of 16 per thread and three.  Included by
+// line_fft.cuh, whose kernels (and those of line_fft_pipe.cuh) take this
+// schedule where is_wide says so.
+//
+// The three-stage kernels move every value through shared memory twice: the
+// L1 / shared-memory pipe ran at 72 to 84% of its peak there while HBM ran at
+// 36 to 55%.  One exchange halves that traffic and its barriers.  A thread
+// holds 32 values (128 registers in all), so 512 threads fill an SM's
+// registers, each with 32 loads in flight.
+//
+// Layout of the exchange: element j of line c at (j + j / R1) * C + c (8
+// lines), so that the two rows a half-warp touches differ in parity in the
+// scatter (rows R1 apart) and in the gather (neighbouring rows); 16 lines are
+// one row per half-warp and need no padding.  With the transposing store the
+// column is XORed with j / 2 (8 lines) or j (16), so that 16 elements along
+// one line spread over all banks.
+#pragma once
+
+namespace agb {
+
+template <int LOGL>
+struct Wide {
+  static_assert(LOGL == 9 || LOGL == 10, "two stages: 16 x 32 or 32 x 32 points");
+  static constexpr int L = 1 << LOGL, E = 32, T = L / E, R1 = L / 32, NSTAGES = 2;
+  static constexpr int twsize() { return 31 * R1; }   // stage 2: W_L^{r k} at [(r - 1) * R1 + k]
+};
+
+template <int LOGL, int C, bool XOR>
+struct WideSmem {
+  static_assert(C == 8 || C == 16, "8 or 16 lines");
+  static constexpr int R1 = Wide<LOGL>::R1;
+  static constexpr int ROWS = Wide<LOGL>::L + (C == 8 ? 32 : 0);
+  static constexpr int FLOAT2S = ROWS * C;
+  float2* s;
+  __device__ __forceinline__ int idx(int c, int j) const {
+    const int row = C == 8 ? j + j / R1 : j;
+    const int col = !XOR ? c : C == 8 ? c ^ ((j >> 1) & 7) : c ^ (j & 15);
+    return row * C + col;
+  }
+  __device__ __forceinline__ void put(int c, int j, float2 v) const { s[idx(c, j)] = v; }
+  __device__ __forceinline__ float2 get(int c, int j) const { return s[idx(c, j)]; }
+};
+
+// W32^k a, k = 0 .. 15
+template <int K>
+__device__ __forceinline__ float2 w32(float2 a) {
+  // cos(pi K / 16)
+  constexpr float cs[17] = {1.f, 0.98078528040323044f, AFFT_C8, 0.83146961230254524f, AFFT_R2, 0.55557023301960218f,
+                            AFFT_S8, 0.19509032201612825f, 0.f, -0.19509032201612825f, -AFFT_S8, -0.55557023301960218f,
+                            -AFFT_R2, -0.83146961230254524f, -AFFT_C8, -0.98078528040323044f, -1.f};
+  if constexpr (K == 0) return a;
+  else if constexpr (K % 2 == 0 && K <= 8) return w16<K / 2>(a);
+  else if constexpr (K == 12) return w16<6>(a);
+  else return cmul(a, make_float2(cs[K], K <= 8 ? -cs[8 - K] : -cs[K - 8]));
+}
+
+template <bool PK, int K>
+__device__ __forceinline__ void dft32_join(float2 (&x)[32], const float2 (&a)[16], const float2 (&b)[16]) {
+  if constexpr (K < 16) {
+    const float2 t = w32<K>(b[K]);
+    x[K] = badd<PK>(a[K], t);
+    x[K + 16] = bsub<PK>(a[K], t);
+    dft32_join<PK, K + 1>(x, a, b);
+  }
+}
+
+// in-place DFT-32, natural order in and out
+template <bool PK>
+__device__ __forceinline__ void dft32(float2 (&x)[32]) {
+  float2 a[16], b[16];
+#pragma unroll
+  for (int i = 0; i < 16; i++) {
+    a[i] = x[2 * i];
+    b[i] = x[2 * i + 1];
+  }
+  dft<16, PK>(a);
+  dft<16, PK>(b);
+  dft32_join<PK, 0>(x, a, b);
+}
+
+// Stage 1 in registers: output r of butterfly b = t + T u (u < 32 / R1) of
+// the canonical values, element b * R1 + r, in v[u + (32 / R1) r].
+template <int LOGL, bool PK>
+__device__ __forceinline__ void wide_stage1(float2 (&v)[32]) {
+  constexpr int R1 = Wide<LOGL>::R1, B1 = 32 / R1;
+#pragma unroll
+  for (int u = 0; u < B1; u++) {
+    float2 x[R1];
+#pragma unroll
+    for (int r = 0; r < R1; r++) x[r] = v[u + B1 * r];
+    if constexpr (R1 == 32) dft32<PK>(x);
+    else dft<16, PK>(x);
+#pragma unroll
+    for (int r = 0; r < R1; r++) v[u + B1 * r] = x[r];
+  }
+}
+
+// Stage 2 on the gathered canonical values (T = R1: butterfly t, k = t)
+template <int LOGL, bool PK>
+__device__ __forceinline__ void wide_stage2(float2 (&v)[32], int t, const float2* tw) {
+  constexpr int R1 = Wide<LOGL>::R1;
+  static_assert(Wide<LOGL>::T == R1, "one stage-2 butterfly per thread");
+#pragma unroll
+  for (int r = 1; r < 32; r++) v[r] = cmul(v[r], ldg2(tw + (r - 1) * R1 + t));
+  dft32<PK>(v);
+}
+
+// Both stages, canonical layout in and out (as run_stages)
+template <int LOGL, bool PK, class SM>
+__device__ __forceinline__ void wide_stages(float2 (&v)[32], int t, int c, const float2* tw, const SM& sm) {
+  constexpr int R1 = Wide<LOGL>::R1, B1 = 32 / R1, T = Wide<LOGL>::T;
+  wide_stage1<LOGL, PK>(v);
+#pragma unroll
+  for (int u = 0; u < B1; u++)
+#pragma unroll
+    for (int r = 0; r < R1; r++) sm.put(c, (t + T * u) * R1 + r, v[u + B1 * r]);
+  __syncthreads();
+#pragma unroll
+  for (int e = 0; e < 32; e++) v[e] = sm.get(c, t + T * e);
+  wide_stage2<LOGL, PK>(v, t, tw);
+}
+
+}  // namespace agb

@@ -39,7 +39,8 @@ template <int... Ls>
 constexpr int stage_total(std::integer_sequence<int, Ls...>) {
   return (Sched<Ls>::twsize() + ... + 0);
 }
-constexpr int kStageTotal = stage_total(std::make_integer_sequence<int, kNoallocLineMaxLog + 1>{});
+constexpr int kStageTotal = stage_total(std::make_integer_sequence<int, kNoallocLineMaxLog + 1>{}) +
+                            Wide<9>::twsize() + Wide<10>::twsize();
 
 static __device__ __align__(256) float g_noalloc_scratch[2 * kNoallocMaxElems];
 static __device__ __align__(256) float2 g_noalloc_stage[kStageTotal + 1];
@@ -52,7 +53,7 @@ struct NoallocDevice {
   float2* stage = nullptr;
   float2* hi = nullptr;
   float2* lo = nullptr;
-  int stage_off[kNoallocLineMaxLog + 1] = {0};
+  int stage_off[kWideTable + kNoallocLineMaxLog] = {0};   // by LineKernel::stage_logl
   int lo_bits[kNoallocMaxLog + 1] = {0};
 };
 
@@ -68,7 +69,8 @@ static int noalloc_setup(int dev, NoallocDevice** out) {
   NoallocDevice& D = g_noalloc_dev[dev];
   if (!D.ready) {
     std::vector<float2> stage;
-    for (int l = 0; l <= kNoallocLineMaxLog; l++) {
+    for (int l = 0; l <= kWideTable + 10; l++) {
+      if (l > kNoallocLineMaxLog && l < kWideTable + 9) continue;   // (the wide tables: 2^9 and 2^10 points)
       D.stage_off[l] = (int)stage.size();
       std::vector<float2> t = stage_table_host(l);
       stage.insert(stage.end(), t.begin(), t.end());
@@ -161,7 +163,7 @@ extern "C" int afft_gb300_c2c_noalloc(const float* src_re, const float* src_im, 
     LineParams p = op.p;
     p.in = noalloc_bind(op.in, base);
     p.out = noalloc_bind(op.out, base);
-    p.tw = D->stage + D->stage_off[op.k.logl];
+    p.tw = D->stage + D->stage_off[op.k.stage_logl];
     if (p.tw_n) {
       p.tw_full = nullptr;   // the static tables are the hi/lo pair
       p.tw_hi = D->hi + (size_t)(lN - kNoallocMinLog) * 2048;

@@ -142,7 +142,18 @@ static std::vector<float2> stage_table_dispatch(int logl, std::integer_sequence<
   return out;
 }
 
+// The same of the 32-points-per-thread cols kernels (Wide): stage 2's
+// W_L^{r k} at [(r - 1) * R1 + k], R1 = L / 32.
+static std::vector<float2> wide_table(int logl) {
+  const int L = 1 << logl, R1 = L / 32;
+  std::vector<float2> t(31 * R1);
+  for (int r = 1; r < 32; r++)
+    for (int k = 0; k < R1; k++) t[(r - 1) * R1 + k] = root_f((long long)r * k, L);
+  return t;
+}
+
 std::vector<float2> stage_table_host(int logl) {
+  if (logl >= kWideTable) return wide_table(logl - kWideTable);
   return stage_table_dispatch(logl, std::make_integer_sequence<int, 15>{});
 }
 
@@ -158,7 +169,7 @@ void fourstep_table_host(long long N, std::vector<float2>* hi, std::vector<float
 }
 
 const float2* stage_twiddles(int logl) {
-  return cached_table(0, logl, [&] { return stage_table_dispatch(logl, std::make_integer_sequence<int, 15>{}); });
+  return cached_table(0, logl, [&] { return stage_table_host(logl); });
 }
 
 const float2* real_twiddles(long long L) {
@@ -507,14 +518,14 @@ struct Builder {
     // cols passes over split planes: the variant with TMA-loaded input tiles
     // (taken at launch when the bound arrays meet its alignment rules)
     if (AFFT_COLS_TMA && !f64 && !tc && cols && !tune.cols_lsu && (kind == LK_C2C || kind == LK_R2C || kind == LK_C2R) &&
-        (!tstore || kind == LK_C2C) && (cpairs == 0 || (cpairs & 1))) {
+        (!tstore || kind == LK_C2C)) {
       LineKernel kt;
       // (the 2048-point R2C pass: unsplit, one CTA per tile, replacing the
       // split form; its LSU kernel is the fallback)
       // (kernels compare by shape: each translation unit has its own host
       // stub of a template kernel, so their addresses differ)
       const bool want = logl < 11 || (kind == LK_C2C ? AFFT_TMA_C2C11 : kind == LK_R2C ? AFFT_TMA_R2C11 : AFFT_TMA_C2R11);
-      const bool have = (cpairs & 1) ? AFFT_TMA_PAIRS && get_cols_tma_pairs(logl, tstore, cpairs, &kt)
+      const bool have = cpairs ? AFFT_TMA_PAIRS && get_cols_tma_pairs(logl, tstore, cpairs, &kt)
                         : tstore   ? AFFT_TMA_TSTORE && get_cols_tma_tstore(logl, &kt)
                                    : get_cols_tma(logl, kind, &kt);
       if (want && have && kt.kind == op.k.kind && kt.logl == op.k.logl && kt.unit == op.k.unit &&
@@ -1237,11 +1248,15 @@ int Plan::launch(const float* src_re, const float* src_im, float* dst_re, float*
       PairedTma pt;
       // (1024-point tiles take the pipelined kernel from two per CTA slot:
       // with one each it has nothing to prefetch and its float exchange
-      // costs more, 2048² c2r 0.0324 vs 0.0300 ms)
+      // costs more, 2048² c2r 0.0324 vs 0.0300 ms; the complex pass up to ten
+      // per slot, arrays that mostly stay in L2: 2^20 x 16 c2c 114 vs 119 us,
+      // but x 64 450 vs 419 and 1024² x 64 397 vs 365, where the CTAs' fixed
+      // shares of the tiles end unevenly)
       const long long slots = (long long)sm_count * op.k.pipe_ctas;
       if (op.k.paired_tma && tma_paired(p, op.k, &pt)) {
         launch_pass(op.k.paired_tma, op.grid, op.threads, op.k.paired_smem, st, p, pt);
-      } else if (op.k.pipe && sm_count > 0 && (op.k.logl == 11 || op.grid >= 2 * slots) && tma_tile(p, op.k, &tm) &&
+      } else if (op.k.pipe && sm_count > 0 && (op.k.logl == 11 || (op.grid >= 2 * slots && (op.k.kind != LK_C2C || op.grid <= 10 * slots))) &&
+          tma_tile(p, op.k, &tm) &&
           (!(AFFT_PIPE_BULK_STORE && !op.k.tstore &&
              ((op.k.kind == LK_C2C && (op.k.logl == 11 || AFFT_PIPE_BULK10)) ||
               (op.k.kind == LK_C2R && op.k.logl == 10 && AFFT_PIPE_BULK_C2R10))) ||

@@ -181,6 +181,10 @@ static int build_queue(QueueImpl& Q) {
       if (op.type == OP_LINE) {
         Segment s;
         s.p = op.p;
+        if (op.k.stage_logl >= kWideTable && !(s.p.tw = stage_twiddles(op.k.stage_logl - kWideTable))) {
+          set_error(AFFT_GB300_ENOMEM, "twiddle table allocation failed");
+          return AFFT_GB300_ENOMEM;
+        }
         s.p.in = bind_io(op.in, base);
         s.p.out = bind_io(op.out, base);
         s.cta0 = op.grid;  // for now the segment's CTA count
@@ -236,8 +240,8 @@ static int build_queue(QueueImpl& Q) {
       g.total = acc;
       host = g.segs.data();
       bytes = g.segs.size() * sizeof(Segment);
-      g.threads = g.k.threads;
-      g.smem = g.pipe ? g.k.pipe_smem : g.k.smem;
+      g.threads = g.pipe ? g.k.threads : g.k.grouped_threads;
+      g.smem = g.pipe ? g.k.pipe_smem : g.k.grouped_smem;
       if (g.smem > 48 * 1024 &&
           cudaFuncSetAttribute((const void*)g.k.grouped, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)g.smem) != cudaSuccess) {
