@@ -469,6 +469,18 @@ __device__ __forceinline__ void line_stages(float2 (&v)[E], int t, int c, const 
   else run_stages<LOGL, C, COLS, WARP_ONLY, 0, TC, packed_bfly<LOGL, COLS, TSTORE>()>(v, t, c, tw, sm, ts);
 }
 
+// The real forward post-pass on a pair of bins (onedim.hpp:1058-1108 /
+// multi.hpp:354-414): X[k] = a - i b, a = (Z[k] + conj Z[L-k]) / 2,
+// b = (Z[k] - conj Z[L-k]) w_k / 2.  The mirror's a and b are the conjugates,
+// so one product serves both: X[L-k] = conj(a + i b).
+__device__ __forceinline__ void post_pair(float2 s0, float2 s1, float2 w, float2& xk, float2& xl) {
+  const float2 a = make_float2(0.5f * (s0.x + s1.x), 0.5f * (s0.y - s1.y));
+  const float2 d = make_float2(0.5f * (s0.x - s1.x), 0.5f * (s0.y + s1.y));
+  const float2 b = cmul(d, w);
+  xk = make_float2(a.x + b.y, a.y - b.x);
+  xl = make_float2(a.x - b.y, -(a.y + b.x));
+}
+
 // The real forward (R2C) pass along a strided axis of Z = 2 Lh complex
 // points (Lh = 2^LOGL), split over two CTAs per tile of C lines.  With the
 // first radix-2 step of a decimation in frequency,
@@ -519,33 +531,35 @@ __device__ __forceinline__ void r2c_half_body(const LineParams& p, long long cta
   // pass below: X[k] = a - i b, X[0] and X[L] from Z[0])
   if constexpr (Sc::NSTAGES > 1) line_sync<WARP_ONLY>();
 #pragma unroll
-  for (int e = 0; e < E; e++) sm.put(c, t + T * e, v[e]);
+  for (int e = E / 2; e < E; e++) sm.put(c, t + T * e, v[e]);
   line_sync<WARP_ONLY>();
   if (active) {
     const long long base = line_off(p.out, q);
     const long long S2 = 2LL * T * p.out.es;
     float* pr = p.out.re + base + (long long)(2 * t + h) * p.out.es;
     float* pi = p.out.im + base + (long long)(2 * t + h) * p.out.es;
+    float* qr = p.out.re + base + (long long)(L - 2 * t - h) * p.out.es;   // bin L - k
+    float* qi = p.out.im + base + (long long)(L - 2 * t - h) * p.out.es;
 #pragma unroll
-    for (int e = 0; e < E; e++) {
+    for (int e = 0; e < E / 2; e++) {
       const int m = t + T * e;
       const int k = 2 * m + h;
       const float2 s0 = v[e];
-      const float2 s1 = sm.get(c, h ? (Lh - 1 - m) : ((Lh - m) & (Lh - 1)));
-      float2 x;
-      if (k == 0) {
-        x = make_float2(s0.x + s0.y, 0.f);
-        const long long aL = base + (long long)L * p.out.es;
-        p.out.re[aL] = s0.x - s0.y;
-        p.out.im[aL] = 0.f;
+      if (k == 0) {   // X[0] and X[L] from Z[0]; X[L/2] = conj(Z[L/2])
+        pr[0] = s0.x + s0.y;
+        pi[0] = 0.f;
+        qr[0] = s0.x - s0.y;
+        qi[0] = 0.f;
+        pr[(E / 2) * S2] = v[E / 2].x;
+        pi[(E / 2) * S2] = -v[E / 2].y;
       } else {
-        const float2 w = ldg2(p.rtw + k);
-        const float2 a = make_float2(0.5f * (s0.x + s1.x), 0.5f * (s0.y - s1.y));
-        const float2 d = make_float2(0.5f * (s0.x - s1.x), 0.5f * (s0.y + s1.y));
-        x = cadd(a, cmul_negi(cmul(d, w)));
+        float2 xk, xl;
+        post_pair(s0, sm.get(c, Lh - h - m), ldg2(p.rtw + k), xk, xl);
+        pr[e * S2] = xk.x;
+        pi[e * S2] = xk.y;
+        qr[-e * S2] = xl.x;
+        qi[-e * S2] = xl.y;
       }
-      pr[e * S2] = x.x;
-      pi[e * S2] = x.y;
     }
   }
 }
@@ -627,34 +641,41 @@ __device__ __forceinline__ void r2c_paired_body(const LineParams& p, long long c
   }
   run_stages<LOGL, C, true, false, 0>(v, t, c, p.tw, sm);
 
+  // A pair of bins at a time: k2 from the lower half of this slot's column
+  // and its mirror, element L2 - 1 - k2 of the partner's (column 0, and the
+  // self-paired column L1/2, within themselves).
   if constexpr (Sc::NSTAGES > 1) __syncthreads();
 #pragma unroll
-  for (int e = 0; e < E; e++) sm.put(c, t + T * e, v[e]);
+  for (int e = E / 2; e < E; e++) sm.put(c, t + T * e, v[e]);
   __syncthreads();
   const long long base = line_off(p.out, q);
+  const long long mbase = line_off(p.out, o * L1 + (k1 == 0 ? 0 : L1 - k1));
+  const int j0 = k1 == 0 ? L2 : L2 - 1;   // the mirror of element k2 is element j0 - k2
   const long long SO = (long long)T * p.out.es;
   float* por = p.out.re + base + (long long)t * p.out.es;
   float* poi = p.out.im + base + (long long)t * p.out.es;
+  float* mor = p.out.re + mbase + (long long)(j0 - t) * p.out.es;
+  float* moi = p.out.im + mbase + (long long)(j0 - t) * p.out.es;
 #pragma unroll
-  for (int e = 0; e < E; e++) {
+  for (int e = 0; e < E / 2; e++) {
     const int k2 = t + T * e;
     const long long k = k1 + L1 * k2;
     const float2 s0 = v[e];
-    const float2 s1 = sm.get(cp, k1 == 0 ? ((L2 - k2) & (L2 - 1)) : (L2 - 1 - k2));
-    float2 x;
-    if (k == 0) {
-      x = make_float2(s0.x + s0.y, 0.f);
-      const long long aL = base + (long long)L2 * p.out.es;
-      p.out.re[aL] = s0.x - s0.y;
-      p.out.im[aL] = 0.f;
+    if (k == 0) {   // X[0] and X[L] (element L2) from Z[0]; X[L/2] = conj(Z[L/2]) (element L2/2 of column 0)
+      por[0] = s0.x + s0.y;
+      poi[0] = 0.f;
+      mor[0] = s0.x - s0.y;
+      moi[0] = 0.f;
+      por[(E / 2) * SO] = v[E / 2].x;
+      poi[(E / 2) * SO] = -v[E / 2].y;
     } else {
-      const float2 w = ldg2(p.rtw + k);
-      const float2 ha = make_float2(0.5f * (s0.x + s1.x), 0.5f * (s0.y - s1.y));
-      const float2 d = make_float2(0.5f * (s0.x - s1.x), 0.5f * (s0.y + s1.y));
-      x = cadd(ha, cmul_negi(cmul(d, w)));
+      float2 xk, xl;
+      post_pair(s0, sm.get(cp, j0 - k2), ldg2(p.rtw + k), xk, xl);
+      por[e * SO] = xk.x;
+      poi[e * SO] = xk.y;
+      mor[-e * SO] = xl.x;
+      moi[-e * SO] = xl.y;
     }
-    por[e * SO] = x.x;
-    poi[e * SO] = x.y;
   }
 }
 
@@ -1392,11 +1413,17 @@ __device__ __forceinline__ void line_fft_body(const LineParams& p, long long cta
     // real forward post-pass (onedim.hpp:1058-1108 / multi.hpp:354-414):
     // X[k] = a - i*b, a = (Z[k] + conj(Z[L-k]))/2,
     // b = (Z[k] - conj(Z[L-k])) * w_k / 2; X[0], X[L] from Z[0].
+    // Warp-staged rows keep one bin per value (the staging takes the
+    // canonical layout); the others take a pair of bins at a time, k from the
+    // lower half of the line and L-k: half the values through shared memory,
+    // half the twiddles and products.
+    constexpr bool STAGED = !COLS && T <= AFFT_STAGE_T && E == 16 && !TC;
+    constexpr int E0 = STAGED || E == 1 ? 0 : E / 2;
     if constexpr (Sc::NSTAGES > 1) line_sync<WARP_ONLY>();
 #pragma unroll
-    for (int e = 0; e < E; e++) sm.put(c, t + T * e, v[e]);
+    for (int e = E0; e < E; e++) sm.put(c, t + T * e, v[e]);
     line_sync<WARP_ONLY>();
-    if constexpr (!COLS && T <= AFFT_STAGE_T && E == 16 && !TC) {
+    if constexpr (STAGED) {
       // bins X[k] (k = t + T e) replace v; xl = X[L] (from the k = 0 thread)
       float2 xl = make_float2(0.f, 0.f);
 #pragma unroll
@@ -1436,32 +1463,33 @@ __device__ __forceinline__ void line_fft_body(const LineParams& p, long long cta
           p.out.im[aL] = xl.y;
         }
       }
-    } else {
-      if (active) {
-        const long long base = line_off(p.out, q);
-        const long long S = (long long)T * p.out.es;
-        float* pr = p.out.re + base + (long long)t * p.out.es;
-        float* pi = p.out.im + base + (long long)t * p.out.es;
+    } else if (active) {
+      const long long base = line_off(p.out, q);
+      const long long S = (long long)T * p.out.es;
+      float* pr = p.out.re + base + (long long)t * p.out.es;
+      float* pi = p.out.im + base + (long long)t * p.out.es;
+      float* qr = p.out.re + base + (long long)(L - t) * p.out.es;   // bin L - k
+      float* qi = p.out.im + base + (long long)(L - t) * p.out.es;
 #pragma unroll
-        for (int e = 0; e < E; e++) {
-          const int k = t + T * e;
-          const float2 s0 = v[e];
-          const float2 s1 = sm.get(c, (L - k) & (L - 1));
-          float2 x;
-          if (k == 0) {
-            x = make_float2(s0.x + s0.y, 0.f);
-            const long long aL = base + (long long)L * p.out.es;
-            p.out.re[aL] = s0.x - s0.y;
-            p.out.im[aL] = 0.f;
-          } else {
-            const float2 w = ldg2(p.rtw + k);
-            const float2 a = make_float2(0.5f * (s0.x + s1.x), 0.5f * (s0.y - s1.y));
-            const float2 d = make_float2(0.5f * (s0.x - s1.x), 0.5f * (s0.y + s1.y));
-            const float2 b = cmul(d, w);
-            x = cadd(a, cmul_negi(b));
+      for (int e = 0; e < (E > 1 ? E / 2 : 1); e++) {
+        const int k = t + T * e;
+        const float2 s0 = v[e];
+        if (k == 0) {   // X[0] and X[L] from Z[0]; X[L/2] = conj(Z[L/2])
+          pr[0] = s0.x + s0.y;
+          pi[0] = 0.f;
+          qr[0] = s0.x - s0.y;
+          qi[0] = 0.f;
+          if constexpr (E > 1) {
+            pr[(E / 2) * S] = v[E / 2].x;
+            pi[(E / 2) * S] = -v[E / 2].y;
           }
-          pr[e * S] = x.x;
-          pi[e * S] = x.y;
+        } else {
+          float2 xk, xl;
+          post_pair(s0, sm.get(c, L - k), ldg2(p.rtw + k), xk, xl);
+          pr[e * S] = xk.x;
+          pi[e * S] = xk.y;
+          qr[-e * S] = xl.x;
+          qi[-e * S] = xl.y;
         }
       }
     }
