@@ -1,4 +1,4 @@
-// Cols passes of 512 and 1024 points with 32 points per thread and two stages
+// Passes of 512 and 1024 points with 32 points per thread and two stages
 // (16 or 32, then 32 points) instead of 16 per thread and three.  Included by
 // line_fft.cuh, whose kernels (and those of line_fft_pipe.cuh) take this
 // schedule where is_wide says so.
@@ -38,6 +38,17 @@ struct WideSmem {
     const int col = !XOR ? c : C == 8 ? c ^ ((j >> 1) & 7) : c ^ (j & 15);
     return row * C + col;
   }
+  __device__ __forceinline__ void put(int c, int j, float2 v) const { s[idx(c, j)] = v; }
+  __device__ __forceinline__ float2 get(int c, int j) const { return s[idx(c, j)]; }
+};
+
+// Rows mode: line c at c * LP, element j at j + j / R1: a half-warp's 16
+// consecutive threads of one line scatter R1 + 1 apart and gather side by side.
+template <int LOGL, int C>
+struct WideRowSmem {
+  static constexpr int R1 = Wide<LOGL>::R1, LP = Wide<LOGL>::L + 32, FLOAT2S = C * LP;
+  float2* s;
+  __device__ __forceinline__ int idx(int c, int j) const { return c * LP + j + j / R1; }
   __device__ __forceinline__ void put(int c, int j, float2 v) const { s[idx(c, j)] = v; }
   __device__ __forceinline__ float2 get(int c, int j) const { return s[idx(c, j)]; }
 };
@@ -107,7 +118,7 @@ __device__ __forceinline__ void wide_stage2(float2 (&v)[32], int t, const float2
 }
 
 // Both stages, canonical layout in and out (as run_stages)
-template <int LOGL, bool PK, class SM>
+template <int LOGL, bool PK, bool WARP_ONLY, class SM>
 __device__ __forceinline__ void wide_stages(float2 (&v)[32], int t, int c, const float2* tw, const SM& sm) {
   constexpr int R1 = Wide<LOGL>::R1, B1 = 32 / R1, T = Wide<LOGL>::T;
   wide_stage1<LOGL, PK>(v);
@@ -115,7 +126,7 @@ __device__ __forceinline__ void wide_stages(float2 (&v)[32], int t, int c, const
   for (int u = 0; u < B1; u++)
 #pragma unroll
     for (int r = 0; r < R1; r++) sm.put(c, (t + T * u) * R1 + r, v[u + B1 * r]);
-  __syncthreads();
+  line_sync<WARP_ONLY>();
 #pragma unroll
   for (int e = 0; e < 32; e++) v[e] = sm.get(c, t + T * e);
   wide_stage2<LOGL, PK>(v, t, tw);

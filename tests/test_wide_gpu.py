@@ -70,6 +70,17 @@ def test_wide(kind, dims, batch, fmt, off):
     check(kind, dims, batch, fmt, off)
 
 
+# rows: whole and partial CTAs (8 and 4 lines each)
+@pytest.mark.parametrize("off", [0, 1])
+@pytest.mark.parametrize("fmt", [0, 1])
+@pytest.mark.parametrize("kind,dims,batch", [
+    ("c", [512], 1), ("ci", [512], 7), ("c", [512], 8), ("c", [512], 1001), ("c", [1024], 1), ("ci", [1024], 3),
+    ("c", [1024], 4), ("ci", [1024], 1001), ("r", [2048], 1), ("r", [2048], 3), ("r", [2048], 1001), ("r", [1024], 5),
+    ("c", [4, 512], 3), ("ci", [8, 1024], 3)])
+def test_rows(kind, dims, batch, fmt, off):
+    check(kind, dims, batch, fmt, off)
+
+
 # 8-line tiles per launch on 304 CTA slots: one below and at two per slot, ten
 # and one tile more
 @pytest.mark.parametrize("kind,dims,batch", [

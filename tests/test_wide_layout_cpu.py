@@ -52,6 +52,20 @@ def test_positions_and_banks(logl, C, xor):
                 assert len(np.unique(half % 16)) == 16
 
 
+@pytest.mark.parametrize("logl", [9, 10])
+def test_rows(logl):
+    L, T = 1 << logl, (1 << logl) // 32
+    C = 128 // T
+    pos = lambda c, j: c * (L + 32) + j + j // T  # noqa: E731  (T = R1)
+    c, j = np.meshgrid(np.arange(C), np.arange(L))
+    p = pos(c.ravel(), j.ravel())
+    assert len(np.unique(p)) == L * C and p.max() < C * (L + 32)
+    tid = np.arange(T * C)
+    for acc in accesses(logl, C):
+        for half in pos(tid // T, acc(tid % T)).reshape(-1, 16):
+            assert len(np.unique(half % 16)) == 16
+
+
 def test_pipelined_1024():
     T, C = 32, 8
     tid = np.arange(T * C)
