@@ -358,31 +358,43 @@ __device__ __forceinline__ void line_fx64_body(const LineParams& p, long long ct
 
   fxc v[E];
   if constexpr (KIND == LK_C2R) {
-    // Z'[i] = a - i*b as line_fft64_body, |Z'| up to four times the bins: two bits lower
+    // Z'[i] = a - i*b as line_fft64_body, |Z'| up to four times the bins: two
+    // bits lower.  A pair of bins at a time, i from the lower half of the line
+    // and L - i, whose a and b are the conjugates: Z'[L-i] = conj(a + i b).
+    // The upper half's bins go through shared memory and its Z' come back the
+    // same way (element L - i is this thread's alone in between).
     sc += 2;
 #pragma unroll
-    for (int e = 0; e < E; e++) {
+    for (int e = 0; e < E; e++) v[e] = {fx_from<TOP - 2>(d[e].x, emax), fx_from<TOP - 2>(d[e].y, emax)};
+#pragma unroll
+    for (int e = E / 2; e < E; e++) sm.put(c, t + T * e, v[e]);
+    line_sync<WARP_ONLY>();
+#pragma unroll
+    for (int e = 0; e < E / 2; e++) {
       const int i = t + T * e;
-      const fxc s0 = {fx_from<TOP - 2>(d[e].x, emax), fx_from<TOP - 2>(d[e].y, emax)};
-      fxc z;
-      if (i == 0) {
+      fxc z, zl;
+      if (i == 0) {   // from the real parts of X[0] and X[L]; Z'[L/2] = 2 conj(X[L/2])
         const fx r1 = fx_from<TOP - 2>(dL, emax);
-        z = {s0.x + r1, s0.x - r1};
+        z = {v[0].x + r1, v[0].x - r1};
+        zl = {2 * v[E / 2].x, -2 * v[E / 2].y};
       } else {
-        fxc s1 = {0, 0};
-        if (active) {
-          const long long a1 = base + (long long)(L - i) * p.in.es;
-          s1 = {fx_from<TOP - 2>(ldd(p.in.re, a1), emax), fx_from<TOP - 2>(ldd(p.in.im, a1), emax)};
-        }
+        const fxc s0 = v[e], s1 = sm.get(c, L - i);
         int4 w = __ldg(rtw + i);
         w.z = -w.z;
         w.w = -w.w;
         const fxc a = {s0.x + s1.x, s0.y - s1.y};
         const fxc b = fx_cmul<true>({s1.x - s0.x, -s1.y - s0.y}, w);
         z = csub_i(a, b);
+        zl = cadd_i(a, b);
+        zl.y = -zl.y;
       }
       v[e] = {z.y, z.x};
+      sm.put(c, i == 0 ? L / 2 : L - i, {zl.y, zl.x});
     }
+    line_sync<WARP_ONLY>();
+#pragma unroll
+    for (int e = E / 2; e < E; e++) v[e] = sm.get(c, t + T * e);
+    line_sync<WARP_ONLY>();   // before the stages write the buffer
   } else {
 #pragma unroll
     for (int e = 0; e < E; e++) {
@@ -416,31 +428,36 @@ __device__ __forceinline__ void line_fx64_body(const LineParams& p, long long ct
       }
     }
   } else if constexpr (KIND == LK_R2C) {
-    // real forward post-pass as line_fft64_body
+    // real forward post-pass as line_fft64_body, a pair of bins at a time (k
+    // from the lower half of the line, and L - k: X[L-k] = conj(h + i b))
     if constexpr (Sc::NSTAGES > 1) line_sync<WARP_ONLY>();
 #pragma unroll
-    for (int e = 0; e < E; e++) sm.put(c, t + T * e, v[e]);
+    for (int e = E / 2; e < E; e++) sm.put(c, t + T * e, v[e]);
     line_sync<WARP_ONLY>();
     if (active) {
       const long long ob = line_off(p.out, q);
       const int sc20 = sc * (1 << 20);
-#pragma unroll
-      for (int e = 0; e < E; e++) {
-        const int k = t + T * e;
-        const fxc s0 = v[e], s1 = sm.get(c, (L - k) & (L - 1));
+      auto emit = [&](int k, fxc x) {
         const long long a = ob + (long long)k * p.out.es;
-        if (k == 0) {
-          const long long aL = ob + (long long)L * p.out.es;
-          std_(p.out.re, aL, fx_to(s0.x - s0.y, sc20));
-          std_(p.out.im, aL, 0.0);
-          std_(p.out.re, a, fx_to(s0.x + s0.y, sc20));
-          std_(p.out.im, a, 0.0);
+        std_(p.out.re, a, fx_to(x.x, sc20));
+        std_(p.out.im, a, fx_to(x.y, sc20));
+      };
+#pragma unroll
+      for (int e = 0; e < E / 2; e++) {
+        const int k = t + T * e;
+        const fxc s0 = v[e];
+        if (k == 0) {   // X[0] and X[L] from Z[0]; X[L/2] = conj(Z[L/2])
+          emit(0, {s0.x + s0.y, 0});
+          emit(L, {s0.x - s0.y, 0});
+          emit(L / 2, {v[E / 2].x, -v[E / 2].y});
         } else {
+          const fxc s1 = sm.get(c, L - k);
           const fxc h = {fx_sar(s0.x + s1.x, 1), fx_sar(s0.y - s1.y, 1)};
           const fxc g = {fx_sar(s0.x - s1.x, 1), fx_sar(s0.y + s1.y, 1)};
-          const fxc x = csub_i(h, fx_cmul<true>(g, __ldg(rtw + k)));
-          std_(p.out.re, a, fx_to(x.x, sc20));
-          std_(p.out.im, a, fx_to(x.y, sc20));
+          const fxc b = fx_cmul<true>(g, __ldg(rtw + k));
+          const fxc y = cadd_i(h, b);
+          emit(k, csub_i(h, b));
+          emit(L - k, {y.x, -y.y});
         }
       }
     }
