@@ -192,7 +192,7 @@ __device__ __forceinline__ void pipe_stages(float2 (&v)[PipeSched<LOGL>::E], int
   if constexpr (LOGL == 10) {
     wide_stage1<LOGL, true>(v);
     pipe_exchange<LOGL, C, 0, KIND == LK_R2C || XOUT>(v, t, c, xs, hook);
-    wide_stage2<LOGL, true>(v, t, tw);
+    wide_last<LOGL, true>(v, t, tw);
   } else if constexpr (S < Sc::NSTAGES) {
     constexpr int R = Sc::radix(S), NS = Sc::ns(S);
     // the butterflies with their outputs kept in registers (stage()'s last-stage form)

@@ -1,5 +1,6 @@
 // Passes of 512 and 1024 points with 32 points per thread and two stages
-// (16 or 32, then 32 points) instead of 16 per thread and three.  Included by
+// (16 or 32, then 32 points) instead of 16 per thread and three, and rows of
+// 8192 and 16384 points with three stages (8 or 16, 32, 32) instead of four.  Included by
 // line_fft.cuh, whose kernels (and those of line_fft_pipe.cuh) take this
 // schedule where is_wide says so.
 //
@@ -21,9 +22,15 @@ namespace agb {
 
 template <int LOGL>
 struct Wide {
-  static_assert(LOGL == 9 || LOGL == 10, "two stages: 16 x 32 or 32 x 32 points");
-  static constexpr int L = 1 << LOGL, E = 32, T = L / E, R1 = L / 32, NSTAGES = 2;
-  static constexpr int twsize() { return 31 * R1; }   // stage 2: W_L^{r k} at [(r - 1) * R1 + k]
+  static_assert(LOGL == 9 || LOGL == 10 || LOGL == 13 || LOGL == 14,
+                "16 x 32, 32 x 32, 8 x 32 x 32 or 16 x 32 x 32 points");
+  static constexpr int L = 1 << LOGL, E = 32, T = L / E, NSTAGES = LOGL <= 10 ? 2 : 3;
+  static constexpr int R1 = LOGL <= 10 ? L / 32 : L / 1024;   // first stage's radix; the others are 32
+  static constexpr int radix(int s) { return s == 0 ? R1 : 32; }
+  static constexpr int ns(int s) { return s == 0 ? 1 : s == 1 ? R1 : 32 * R1; }
+  // stage twiddles as Sched's: W_{NS R}^{r k} at [twoff(s) + (r - 1) * NS + k]
+  static constexpr int twoff(int s) { return s <= 1 ? 0 : 31 * R1; }
+  static constexpr int twsize() { return NSTAGES == 2 ? 31 * R1 : 31 * R1 * 33; }
 };
 
 template <int LOGL, int C, bool XOR>
@@ -42,13 +49,20 @@ struct WideSmem {
   __device__ __forceinline__ float2 get(int c, int j) const { return s[idx(c, j)]; }
 };
 
-// Rows mode: line c at c * LP, element j at j + j / R1: a half-warp's 16
-// consecutive threads of one line scatter R1 + 1 apart and gather side by side.
+// Rows mode: line c at c * LP.  Two stages: element j at j + j / R1, a
+// half-warp's 16 consecutive threads of one line scatter R1 + 1 apart and gather
+// side by side.  Three stages: j + j / 16 + 8 (j / 256), conflict-free for the
+// first stage's scatter (stride 8 or 16), the second's (8 or 16 neighbours,
+// groups of 8 going 256 apart) and the gather.
 template <int LOGL, int C>
 struct WideRowSmem {
-  static constexpr int R1 = Wide<LOGL>::R1, LP = Wide<LOGL>::L + 32, FLOAT2S = C * LP;
+  static constexpr int R1 = Wide<LOGL>::R1, L = Wide<LOGL>::L;
+  static constexpr int LP = LOGL <= 10 ? L + 32 : L + L / 16 + 8 * (L / 256), FLOAT2S = C * LP;
   float2* s;
-  __device__ __forceinline__ int idx(int c, int j) const { return c * LP + j + j / R1; }
+  __device__ __forceinline__ int idx(int c, int j) const {
+    if constexpr (LOGL <= 10) return c * LP + j + j / R1;
+    else return c * LP + j + (j >> 4) + ((j >> 8) << 3);
+  }
   __device__ __forceinline__ void put(int c, int j, float2 v) const { s[idx(c, j)] = v; }
   __device__ __forceinline__ float2 get(int c, int j) const { return s[idx(c, j)]; }
 };
@@ -101,23 +115,23 @@ __device__ __forceinline__ void wide_stage1(float2 (&v)[32]) {
 #pragma unroll
     for (int r = 0; r < R1; r++) x[r] = v[u + B1 * r];
     if constexpr (R1 == 32) dft32<PK>(x);
-    else dft<16, PK>(x);
+    else dft<R1, PK>(x);
 #pragma unroll
     for (int r = 0; r < R1; r++) v[u + B1 * r] = x[r];
   }
 }
 
-// Stage 2 on the gathered canonical values (T = R1: butterfly t, k = t)
+// The last stage on the gathered canonical values (butterfly t, k = t: T = NS)
 template <int LOGL, bool PK>
-__device__ __forceinline__ void wide_stage2(float2 (&v)[32], int t, const float2* tw) {
-  constexpr int R1 = Wide<LOGL>::R1;
-  static_assert(Wide<LOGL>::T == R1, "one stage-2 butterfly per thread");
+__device__ __forceinline__ void wide_last(float2 (&v)[32], int t, const float2* tw) {
+  constexpr int T = Wide<LOGL>::T;
+  static_assert(T == Wide<LOGL>::ns(Wide<LOGL>::NSTAGES - 1), "one last-stage butterfly per thread");
 #pragma unroll
-  for (int r = 1; r < 32; r++) v[r] = cmul(v[r], ldg2(tw + (r - 1) * R1 + t));
+  for (int r = 1; r < 32; r++) v[r] = cmul(v[r], ldg2(tw + (r - 1) * T + t));
   dft32<PK>(v);
 }
 
-// Both stages, canonical layout in and out (as run_stages)
+// All stages, canonical layout in and out (as run_stages)
 template <int LOGL, bool PK, bool WARP_ONLY, class SM>
 __device__ __forceinline__ void wide_stages(float2 (&v)[32], int t, int c, const float2* tw, const SM& sm) {
   constexpr int R1 = Wide<LOGL>::R1, B1 = 32 / R1, T = Wide<LOGL>::T;
@@ -129,7 +143,20 @@ __device__ __forceinline__ void wide_stages(float2 (&v)[32], int t, int c, const
   line_sync<WARP_ONLY>();
 #pragma unroll
   for (int e = 0; e < 32; e++) v[e] = sm.get(c, t + T * e);
-  wide_stage2<LOGL, PK>(v, t, tw);
+  if constexpr (Wide<LOGL>::NSTAGES == 3) {
+    line_sync<WARP_ONLY>();   // every gather is done before the next scatter
+    const int k = t & (R1 - 1);
+#pragma unroll
+    for (int r = 1; r < 32; r++) v[r] = cmul(v[r], ldg2(tw + (r - 1) * R1 + k));
+    dft32<PK>(v);
+    const int base = (t / R1) * (32 * R1) + k;
+#pragma unroll
+    for (int r = 0; r < 32; r++) sm.put(c, base + r * R1, v[r]);
+    line_sync<WARP_ONLY>();
+#pragma unroll
+    for (int e = 0; e < 32; e++) v[e] = sm.get(c, t + T * e);
+  }
+  wide_last<LOGL, PK>(v, t, tw + Wide<LOGL>::twoff(Wide<LOGL>::NSTAGES - 1));
 }
 
 }  // namespace agb

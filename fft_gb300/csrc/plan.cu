@@ -142,18 +142,25 @@ static std::vector<float2> stage_table_dispatch(int logl, std::integer_sequence<
   return out;
 }
 
-// The same of the 32-points-per-thread cols kernels (Wide): stage 2's
-// W_L^{r k} at [(r - 1) * R1 + k], R1 = L / 32.
-static std::vector<float2> wide_table(int logl) {
-  const int L = 1 << logl, R1 = L / 32;
-  std::vector<float2> t(31 * R1);
-  for (int r = 1; r < 32; r++)
-    for (int k = 0; k < R1; k++) t[(r - 1) * R1 + k] = root_f((long long)r * k, L);
+// The same of the 32-points-per-thread kernels (Wide)
+template <int LOGL>
+static std::vector<float2> wide_table() {
+  using S = Wide<LOGL>;
+  std::vector<float2> t(S::twsize());
+  for (int s = 1; s < S::NSTAGES; s++)
+    for (int r = 1; r < 32; r++)
+      for (int k = 0; k < S::ns(s); k++)
+        t[S::twoff(s) + (r - 1) * S::ns(s) + k] = root_f((long long)r * k, 32LL * S::ns(s));
   return t;
 }
 
 std::vector<float2> stage_table_host(int logl) {
-  if (logl >= kWideTable) return wide_table(logl - kWideTable);
+  switch (logl - kWideTable) {
+    case 9: return wide_table<9>();
+    case 10: return wide_table<10>();
+    case 13: return wide_table<13>();
+    case 14: return wide_table<14>();
+  }
   return stage_table_dispatch(logl, std::make_integer_sequence<int, 15>{});
 }
 

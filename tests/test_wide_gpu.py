@@ -76,7 +76,9 @@ def test_wide(kind, dims, batch, fmt, off):
 @pytest.mark.parametrize("kind,dims,batch", [
     ("c", [512], 1), ("ci", [512], 7), ("c", [512], 8), ("c", [512], 1001), ("c", [1024], 1), ("ci", [1024], 3),
     ("c", [1024], 4), ("ci", [1024], 1001), ("r", [2048], 1), ("r", [2048], 3), ("r", [2048], 1001), ("r", [1024], 5),
-    ("c", [4, 512], 3), ("ci", [8, 1024], 3)])
+    ("c", [4, 512], 3), ("ci", [8, 1024], 3),
+    ("c", [8192], 1), ("ci", [8192], 5), ("c", [16384], 1), ("ci", [16384], 3), ("r", [16384], 1), ("r", [16384], 5),
+    ("r", [32768], 3), ("ri", [16384], 3), ("ri", [32768], 3)])
 def test_rows(kind, dims, batch, fmt, off):
     check(kind, dims, batch, fmt, off)
 

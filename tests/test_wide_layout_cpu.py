@@ -66,6 +66,36 @@ def test_rows(logl):
             assert len(np.unique(half % 16)) == 16
 
 
+# 8192- and 16384-point rows: three stages (8 or 16, 32, 32 points)
+@pytest.mark.parametrize("logl", [13, 14])
+def test_long_rows(logl):
+    L, T, r1 = 1 << logl, (1 << logl) // 32, (1 << logl) // 1024
+    pos = lambda j: j + (j >> 4) + ((j >> 8) << 3)  # noqa: E731
+    p = pos(np.arange(L))
+    assert len(np.unique(p)) == L and p.max() < L + L // 16 + 8 * (L // 256)
+    t = np.arange(T)
+    acc = [(t + T * u) * r1 + r for u in range(32 // r1) for r in range(r1)]
+    acc += [(t // r1) * (32 * r1) + t % r1 + r * r1 for r in range(32)] + [t + T * e for e in range(32)]
+    for j in acc:
+        for half in pos(j).reshape(-1, 16):
+            assert len(np.unique(half % 16)) == 16
+    rng = np.random.default_rng(logl)
+    x = rng.standard_normal(L) + 1j * rng.standard_normal(L)
+    b1, b2, out = (np.empty(L, complex) for _ in range(3))
+    for t in range(T):
+        v = x[t + T * np.arange(32)]
+        for u in range(32 // r1):
+            b = t + T * u
+            b1[b * r1:(b + 1) * r1] = np.fft.fft(v[u + (32 // r1) * np.arange(r1)])
+    r = np.arange(32)
+    for t in range(T):
+        k = t % r1
+        b2[(t // r1) * 32 * r1 + k + r * r1] = np.fft.fft(b1[t + T * r] * np.exp(-2j * np.pi * r * k / (32 * r1)))
+    for t in range(T):
+        out[t + T * r] = np.fft.fft(b2[t + T * r] * np.exp(-2j * np.pi * r * t / L))
+    assert np.abs(out - np.fft.fft(x)).max() < 1e-9
+
+
 def test_pipelined_1024():
     T, C = 32, 8
     tid = np.arange(T * C)
