@@ -30,8 +30,9 @@ struct LineKernel {
   int halves;          // CTAs per tile of C lines (2: the split R2C pass)
   int stage_logl;      // log2 length of the stage twiddle table the kernel reads (+ kWideTable: the
                        // table of the 32-points-per-thread schedule)
-  int grouped_threads; // threads, shared memory of the grouped forms (16 points per thread at every length:
-  size_t grouped_smem; // their stage table is the one without kWideTable)
+  int grouped_threads;      // the same of the grouped forms, whose schedule may be the other one
+  size_t grouped_smem;
+  int grouped_stage_logl;
   LineKernelTmaFn tma; // the same pass with its input tile loaded by TMA (cols passes over
                        // split planes), or null
   GroupedKernelFn grouped_tma;   // its grouped form (queue segments with tensor maps), or null
@@ -93,7 +94,7 @@ bool get_cols_tma(int logl, int kind, LineKernel* out);
 bool get_cols_tma_tstore(int logl, LineKernel* out);
 // complex cols passes over interleaved input pairs (pairs bit 0 set: 1 or
 // 3), plain or with the transposing store, 2^8 to 2^10 points, and split input with output pairs
-// (pairs 2, not transposing, 2^9 and 2^10 points), with TMA
+// (pairs 2, not transposing), with TMA
 // loads of the interleaved tile (k_cols_tma_pairs.cu)
 bool get_cols_tma_pairs(int logl, bool tstore, int pairs, LineKernel* out);
 
@@ -190,8 +191,10 @@ LineKernel make_line_kernel() {
   k.lines_per_cta = C;
   k.threads = Sc::T * C;
   k.smem = (size_t)SmemOf<LOGL, C, COLS, KIND, TSTORE, TC>::FLOAT2S * sizeof(float2);
-  k.grouped_threads = Sched<LOGL>::T * C;
-  k.grouped_smem = (size_t)LineSmem<LOGL, C, COLS, TSTORE, TC>::FLOAT2S * sizeof(float2);
+  using Gr = SchedOf<LOGL, COLS, KIND, TC, true>;
+  k.grouped_threads = Gr::T * C;
+  k.grouped_smem = (size_t)SmemOf<LOGL, C, COLS, KIND, TSTORE, TC, true>::FLOAT2S * sizeof(float2);
+  k.grouped_stage_logl = LOGL + (Gr::E == 32 ? kWideTable : 0);
   return k;
 }
 
@@ -246,7 +249,7 @@ LineKernel make_plane_kernel() {
   k.threads = k.grouped_threads = PS::NT;
   k.smem = k.grouped_smem = (size_t)PS::FLOAT2S * sizeof(float2);
   k.halves = 1;
-  k.stage_logl = LOG2;
+  k.stage_logl = k.grouped_stage_logl = LOG2;
   return k;
 }
 

@@ -337,23 +337,25 @@ namespace agb {
 
 // Which kernels take the 32-points-per-thread schedule of line_wide.cuh,
 // against 16 points per thread (us):
-//  - complex and plain real cols passes of 512 and 1024 points and the split 2048-point R2C pass: 2^20
-//    c2c x 16 127 -> 115, x 64 450 -> 420, 1024^2 x 64 368 -> 365, 512^2 x 37
+//  - complex and plain real cols passes of 512 and 1024 points and the split
+//    2048-point R2C pass: 2^20 c2c x 16 127 -> 115, x 64 450 -> 420, 1024^2 x 64 368 -> 365, 512^2 x 37
 //    58.7 -> 57.0 (as pairs 63.5 -> 60.2), 2^20 r2c x 64 300 -> 286, c2r 334 ->
 //    297, 2048^2 c2r x 16 211 -> 192, r2c x 4 65.0 -> 62.2, 4096^2 r2c 74.4 ->
 //    72.8; not the paired real passes (2^20 r2c x 64 286 vs 318);
-//  - complex rows of those lengths, whose lines then sit in a warp or half of one, without CTA
-//    barriers: 1024 x 65536 168 -> 153, as pairs 190 -> 154, 512 x 131072 157 ->
+//  - complex rows of those lengths, whose lines then sit in a warp or half of
+//    one, without CTA barriers: 1024 x 65536 168 -> 153, as pairs 190 -> 154, 512 x 131072 157 ->
 //    154, as pairs 164 -> 154; and the 1024-point rows R2C pass, 2048 reals x
 //    65536 204 -> 170 (the 512-point one 186 -> 191, C2R level);
 //  - complex and R2C rows of 8192 and 16384 points (three stages against four):
 //    8192 x 8192 248 -> 210, as pairs 267 -> 224, 16384 x 4096 332 -> 306, 16384
 //    reals x 8192 304 -> 252; not the C2R rows (350 vs 361);
-//  - not the queue's grouped kernels (GROUPED), which share the SMs with other
-//    groups (1000 mixed transforms 1005 vs 1040).
+//  - of the queue's grouped kernels (GROUPED), which share the SMs with other
+//    groups, only the 1024-point rows (10000 mixed transforms 11.92 -> 11.73 ms,
+//    fewer level); the cols passes there are slower (1000 transforms 1005 vs
+//    1040 us), the other rows level.
 template <int LOGL, bool COLS, int KIND, bool TC, bool GROUPED>
 constexpr bool is_wide() {
-  if (TC || GROUPED) return false;
+  if (TC || (GROUPED && (COLS || LOGL != 10))) return false;
   if (LOGL == 13 || LOGL == 14) return !COLS && (KIND == LK_C2C || KIND == LK_R2C);
   return (LOGL == 9 || LOGL == 10) &&
          (COLS ? KIND <= LK_R2C_HALF : KIND == LK_C2C || (KIND == LK_R2C && LOGL == 10));
@@ -1736,7 +1738,8 @@ __device__ __forceinline__ void stage_params(LineParams& dst, const LineParams& 
 // TMA: every segment has tensor maps and loads its tiles by TMA (as
 // line_fft_tma); segments without them go to the LSU form of the kernel.
 template <int LOGL, int C, bool COLS, int KIND, bool TSTORE, bool TC = false, int UNIT = 0, bool TMA = false>
-__global__ void __launch_bounds__(Sched<LOGL>::T * C, min_ctas<Sched<LOGL>::T * C>())
+__global__ void __launch_bounds__(SchedOf<LOGL, COLS, KIND, TC, true>::T * C,
+                                  cta_bound<SchedOf<LOGL, COLS, KIND, TC, true>, C>())
 line_fft_grouped(const Segment* __restrict__ segs, const int* __restrict__ seg_of, long long total) {
   __shared__ LineParams sp;
   if constexpr (TMA) {

@@ -181,7 +181,7 @@ static int build_queue(QueueImpl& Q) {
       if (op.type == OP_LINE) {
         Segment s;
         s.p = op.p;
-        if (op.k.stage_logl >= kWideTable && !(s.p.tw = stage_twiddles(op.k.stage_logl - kWideTable))) {
+        if (op.k.grouped_stage_logl != op.k.stage_logl && !(s.p.tw = stage_twiddles(op.k.grouped_stage_logl))) {
           set_error(AFFT_GB300_ENOMEM, "twiddle table allocation failed");
           return AFFT_GB300_ENOMEM;
         }
