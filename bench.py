@@ -76,10 +76,8 @@ DIST_TEXT = {"uniform": "seeded uniform[-1,1)", "normal": "seeded standard norma
 
 FORMS = {"plain": "plain FP32 Stockham",
          "tc": "split-precision tensor cores (tcgen05 DFT-16, FP16 hi+lo, FP32 accumulate) where eligible",
-         "f64": "FP64 data and arithmetic (afft_64_*): radix-8 Stockham FP64 kernels"}
+         "f64": "FP64 data (afft_64_*): radix-8 Stockham stages in 64-bit block fixed point"}
 
-# GB300's nominal FP64 rate (GFLOP/s); MEASURED_PEAKS.json has no FP64 figure
-FP64_NOMINAL_GFLOPS = 1250.0
 # GB300 L2 capacity (bytes)
 L2_BYTES = 129e6
 
@@ -543,19 +541,10 @@ def measure_plan(args, cfg, dev, stream, world=1, rank=0, steps=None, soak=None,
               "frac": round(pb / (fwd_ms / 1e3) / 1e9 / hbm, 4), "unit": "GB/s"}
     kernel = "forward plan (%d launch%s), %.4f ms per launch" % (fwd.launches, "es" if fwd.launches > 1 else "",
                                                                   fwd_ms / fwd.launches)
-    if f64:
-        # FP64 arithmetic, not HBM, bounds the FP64 kernels on GB300
-        fwd_gflops = flops_of(kind, dims, batch) / (fwd_ms / 1e3) / 1e9
-        roofline = {"bound": "fp64", "achieved": round(fwd_gflops, 1), "peak": FP64_NOMINAL_GFLOPS,
-                    "unit": "GFLOP/s", "frac": round(fwd_gflops / FP64_NOMINAL_GFLOPS, 4), "traffic": None,
-                    "peak_source": "nominal (no measured FP64 figure)", "kernel": kernel,
-                    "hbm": {"achieved": round(achieved, 1), "peak": hbm, "frac": round(achieved / hbm, 4),
-                            "unit": "GB/s"},
-                    "passes": passes}
-    else:
-        roofline = {"bound": "hbm", "achieved": round(achieved, 1), "peak": hbm, "unit": "GB/s",
-                    "frac": round(achieved / hbm, 4), "traffic": None, "peak_source": peak_src,
-                    "kernel": kernel, "passes": passes}
+    # (FP64 plans too: their stages run on the integer pipes, in block fixed point)
+    roofline = {"bound": "hbm", "achieved": round(achieved, 1), "peak": hbm, "unit": "GB/s",
+                "frac": round(achieved / hbm, 4), "traffic": None, "peak_source": peak_src,
+                "kernel": kernel, "passes": passes}
     rec = {"value": round(value, 2), "unit": "GFLOP/s", "ms_per_step": round(ms_step, 4),
            "ms_per_launch": round(fwd_ms / fwd.launches, 5), "fwd_ms": round(fwd_ms, 5),
            "gbs_algorithmic": round(achieved, 1), "roofline": roofline, "accuracy": acc,

@@ -24,7 +24,7 @@ afft_auto, afft_scalar, afft_sse2, afft_avx2, afft_avx512f, afft_neon, afft_gb30
 afft_split, afft_interleaved = 0, 1
 KIND_C, KIND_CI, KIND_R, KIND_RI = 0, 1, 2, 3
 FORM_TC = 0x100   # AFFT_GB300_FORM_TC: split-precision tensor-core butterflies
-FORM_F64 = 0x200  # AFFT_GB300_FORM_F64: FP64 data and arithmetic (the afft_64_* path)
+FORM_F64 = 0x200  # AFFT_GB300_FORM_F64: FP64 data and accuracy (the afft_64_* path)
 QUEUE_TUNED = 0x400  # AFFT_GB300_QUEUE_TUNED: queue plans take the autotuner's per-shape choices
 KINDS = {"c": KIND_C, "ci": KIND_CI, "r": KIND_R, "ri": KIND_RI}
 ERRORS = {0: "OK", 1: "EINVAL", 2: "ENODEV", 3: "ENOMEM", 4: "ECUDA", 5: "ESTATE", 6: "ETIMEOUT"}
@@ -368,7 +368,7 @@ class BatchPlan:
     """``batch`` dense transforms of one shape and kind (extension).
 
     ``form``: None / "plain" (FP32), "tc" (split-precision tensor cores) or
-    "f64" (double arrays, FP64 arithmetic).  ``__call__`` is synchronous (like
+    "f64" (double arrays, FP64 accuracy).  ``__call__`` is synchronous (like
     afft); ``launch`` enqueues on a CUDA stream (device pointers only) and
     returns immediately.
     """

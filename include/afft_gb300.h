@@ -116,8 +116,9 @@ AFFT_GB300_API void afft_32_ri_transform(afft_32_ri_type* state,
 AFFT_GB300_API size_t afft_32_align_size(size_t sz);
 
 /* Replaces fft.h:48-80 (FP64): the same transforms, layouts, errors and
- * pointer rules on double arrays, computed in FP64 by the library's FP64
- * kernels (twiddles computed in FP64, never rounded).  A plan made by an
+ * pointer rules on double arrays, to FP64 accuracy: lines are transformed in
+ * 64-bit block fixed point (one exponent per line, relative L2 error 1e-16 to
+ * 3e-16), lines that do not fit it on the FP64 pipe.  A plan made by an
  * afft_64_*_create (or a batched plan with AFFT_GB300_FORM_F64) runs only
  * through the afft_64_* transforms, an FP32 plan only through the afft_32_*
  * ones; a mismatch sets AFFT_GB300_EINVAL and launches nothing. */
@@ -188,7 +189,7 @@ enum { afft_gb300_c = 0, afft_gb300_ci = 1, afft_gb300_r = 2, afft_gb300_ri = 3 
 enum { AFFT_GB300_FORM_TC = 0x100 };
 
 /* Form flag, OR-ed into `format` of afft_gb300_batch_memsize/_create and
- * afft_gb300_plan_describe: double arrays and FP64 arithmetic (the batched
+ * afft_gb300_plan_describe: double arrays and FP64 accuracy (the batched
  * form of the afft_64_* transforms; run it with afft_64_<kind>_transform, or
  * with afft_gb300_transform_async passing the double pointers as float*).
  * Not combinable with AFFT_GB300_FORM_TC, and not accepted by the queue. */
