@@ -148,6 +148,26 @@ static size_t memsize_impl(int kind, size_t ndim, const size_t* dim, size_t batc
   return kPlanMem;
 }
 
+// A plan with its device scratch, so later launches allocate nothing (and can
+// be captured into CUDA graphs).  FP64 axes in three passes take twice the
+// scratch of two: where that much is not free, two passes.
+static std::unique_ptr<Plan> build_with_scratch(int kind, int ndim, const long long* dims, long long batch,
+                                                int format, int form) {
+  Tuning two;
+  two.passes = 2;
+  for (const Tuning* t : {(const Tuning*)nullptr, (const Tuning*)&two}) {
+    auto P = build_plan(kind, ndim, dims, batch, format, false, form, t);
+    if (!P) return nullptr;
+    if (P->scratch_elems == 0 || cudaMalloc(&P->scratch, (size_t)P->scratch_elems * P->esize()) == cudaSuccess)
+      return P;
+    cudaGetLastError();
+    P->scratch = nullptr;
+    if (!P->f64()) break;
+  }
+  set_error(AFFT_GB300_ENOMEM, "scratch allocation failed");
+  return nullptr;
+}
+
 static void* create_impl(int kind, size_t ndim, const size_t* dim, size_t batch, int format, void* mem,
                          int impl, int form = 0) {
   int nd;
@@ -158,15 +178,8 @@ static void* create_impl(int kind, size_t ndim, const size_t* dim, size_t batch,
     set_error(AFFT_GB300_EINVAL, "null mem or zero batch");
     return nullptr;
   }
-  auto P = build_plan(kind, nd, dims, (long long)batch, format, false, form);
+  auto P = build_with_scratch(kind, nd, dims, (long long)batch, format, form);
   if (!P) return nullptr;
-  // device scratch now, so later launches allocate nothing (and can be
-  // captured into CUDA graphs)
-  if (P->scratch_elems > 0 && cudaMalloc(&P->scratch, (size_t)P->scratch_elems * P->esize()) != cudaSuccess) {
-    cudaGetLastError();
-    set_error(AFFT_GB300_ENOMEM, "scratch allocation failed");
-    return nullptr;
-  }
   // A blocking stream: the synchronous transform calls are ordered after
   // work the caller queued on the default stream (the input is complete),
   // as afft's synchronous calls read finished data.
@@ -394,8 +407,11 @@ static int transform_sync(void* plan, const float* sr, const float* si, float* d
       for (long long d = 8; d >= 2; d--)
         if (P->batch % d == 0) { k = d; break; }
     if (k > 1) {
-      P->chunk = build_plan(P->kind, P->ndim, P->dims, P->batch / k, P->format, false, P->form);
-      if (!P->chunk) k = 1;
+      P->chunk = build_with_scratch(P->kind, P->ndim, P->dims, P->batch / k, P->format, P->form);
+      if (!P->chunk) {
+        clear_error();
+        k = 1;   // the whole batch at once, on the plan's own scratch
+      }
     }
     // streams and events are set up all or nothing: copy_in, set last,
     // marks them ready

@@ -742,13 +742,13 @@ struct Builder {
     if (a_bs == 0) a_bs = L * inner;
     if (b_bs == 0) b_bs = L * inner;
     int logl = ilog2ll(L);
-    // FP64 lines of 8192 points fill an SM with one CTA, whose stages nothing
-    // overlaps: from 8 lines two passes of 128 and 64 points (2048 lines 404
-    // -> 316 us, 64 lines 28 -> 18), while the scratch they need stays small
     const long long pts = outer * L;
-    const bool split13 = f64 && logl == ROWS_MAX_LOG64 && outer >= 8 && pts <= (1LL << 28);
     if (inner == 1) {
-      if (logl <= rows_max() && !split13) {
+      // (FP64 lines of 8192 points fill an SM with one CTA, whose stages
+      // nothing overlaps; two passes of 128 and 64 points run 2048 lines in
+      // 316 us instead of 404, but through scratch, and a plan without scratch
+      // may run on several streams at once)
+      if (logl <= rows_max()) {
         line(LK_C2C, false, false, logl, io(A, 1, 0, a_bs, 0, 0), io(B, 1, 0, b_bs, 0, 0), outer, inverse);
         return;
       }
@@ -758,8 +758,9 @@ struct Builder {
       // of 1024 / 2048, whose one-CTA-per-SM tiles run at about half the
       // rate per pass
       // (FP64: from 2^20 points a line and 2^23 in all, 16 x 2^20 582 -> 468
-      // us, 4 x 2^22 796 -> 597, 32 x 2^19 513 -> 582; up to 4 GB of scratch)
-      const bool three = f64 ? logl >= 20 && pts >= (1LL << 23) && pts <= (1LL << 27)
+      // us, 4 x 2^22 796 -> 597, 32 x 2^19 513 -> 582; up to 4 GB of scratch,
+      // two passes where the device has not that much left)
+      const bool three = f64 ? tune.passes != 2 && logl >= 20 && pts >= (1LL << 23) && pts <= (1LL << 27)
                              : (tune.passes == 3 ? logl >= 20 : tune.passes == 2 ? false : logl >= AFFT_THREE_PASS_LOG);
       int l1 = three ? 8 : l1_of(logl), l2 = logl - l1;
       if (l1 > COLS_MAX_LOG || (l2 > COLS_MAX_LOG && !three)) {

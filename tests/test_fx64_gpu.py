@@ -85,7 +85,7 @@ def test_strided(dims, dev):
     assert rel(run("c", dims, 1, (a, b), dev), sfft.fftn(z).reshape(1, -1)) <= TOL
 
 
-# lines of 8192 points in two passes, axes of 2^20 points in three
+# lines of 8192 points, the longest of one pass; axes of 2^20 points in three
 @pytest.mark.parametrize("kind,dims,batch", [("c", [8192], 9), ("ci", [2, 8192], 5), ("c", [1 << 20], 8)])
 def test_split_lines(kind, dims, batch, dev):
     rng = np.random.default_rng(5)
