@@ -157,16 +157,22 @@ __device__ __forceinline__ float2 cswap(float2 a) { return make_float2(a.y, a.x)
 #define AFFT_S8 0.38268343236508979f
 #define AFFT_R2 0.70710678118654752f
 
-// W16^k * a for k = 1..9 (forward, exp(-2 pi i k/16))
+// a (x + iy), |x| the larger of the two factors when XL: of each component's
+// two products the one by the smaller factor is rounded by itself
+template <bool XL>
+__device__ __forceinline__ float2 cmulc(float2 a, float x, float y) {
+  if constexpr (XL) return make_float2(fmaf(a.x, x, -a.y * y), fmaf(a.y, x, a.x * y));
+  else return make_float2(fmaf(-a.y, y, a.x * x), fmaf(a.x, y, a.y * x));
+}
+
+// W16^k * a, k = 1, 3, 4, 9 (forward, exp(-2 pi i k/16); the others go by w8s)
 template <int K>
 __device__ __forceinline__ float2 w16(float2 a) {
   if constexpr (K == 0) return a;
-  else if constexpr (K == 1) return cmul(a, make_float2(AFFT_C8, -AFFT_S8));
-  else if constexpr (K == 2) return make_float2(AFFT_R2 * (a.x + a.y), AFFT_R2 * (a.y - a.x));
-  else if constexpr (K == 3) return cmul(a, make_float2(AFFT_S8, -AFFT_C8));
+  else if constexpr (K == 1) return cmulc<true>(a, AFFT_C8, -AFFT_S8);
+  else if constexpr (K == 3) return cmulc<false>(a, AFFT_S8, -AFFT_C8);
   else if constexpr (K == 4) return cmul_negi(a);
-  else if constexpr (K == 6) return make_float2(AFFT_R2 * (a.y - a.x), -AFFT_R2 * (a.x + a.y));
-  else if constexpr (K == 9) return cmul(a, make_float2(-AFFT_C8, AFFT_S8));
+  else if constexpr (K == 9) return cmulc<true>(a, -AFFT_C8, AFFT_S8);
   else return a;  // unused
 }
 
@@ -188,6 +194,51 @@ __device__ __forceinline__ void dft4(float2& a0, float2& a1, float2& a2, float2&
   a3 = bsub<PK>(d02, cmul_negi(d13));
 }
 
+// sqrt(2) W8^K a, K = 1 or 3
+template <int K>
+__device__ __forceinline__ float2 w8s(float2 a) {
+  static_assert(K == 1 || K == 3, "the other powers are 1 and -i");
+  return K == 1 ? make_float2(a.x + a.y, a.y - a.x) : make_float2(a.y - a.x, -a.x - a.y);
+}
+
+// (a, b) = (a + sqrt(1/2) b, a - sqrt(1/2) b): W8's factor in the butterfly's
+// own multiply-add.  Eight multiplies and as many roundings fewer per DFT-16:
+// 8192-point rows 215 -> 206 us (8192 lines), 4096 172.2 -> 170.4 (16384),
+// 2048^2 c2c x 8 229 -> 226, rel-L2 of 4096 points 1.24e-7 -> 1.20e-7; passes
+// that HBM or shared memory bounds are level.
+template <bool PK>
+__device__ __forceinline__ void bf8(float2& a, float2& b) {
+  const float2 t = a;
+  if constexpr (PK) {
+    a = __ffma2_rn(make_float2(AFFT_R2, AFFT_R2), b, t);
+    b = __ffma2_rn(make_float2(-AFFT_R2, -AFFT_R2), b, t);
+  } else {
+    a = make_float2(fmaf(AFFT_R2, b.x, t.x), fmaf(AFFT_R2, b.y, t.y));
+    b = make_float2(fmaf(-AFFT_R2, b.x, t.x), fmaf(-AFFT_R2, b.y, t.y));
+  }
+}
+
+// dft4 whose a2 (E8) or a1 and a3 (O8) still lack the factor sqrt(1/2)
+template <bool PK, bool E8, bool O8>
+__device__ __forceinline__ void dft4_8(float2& a0, float2& a1, float2& a2, float2& a3) {
+  float2 s = a0, m = a2, p = a1, q = a3;
+  if constexpr (E8) bf8<PK>(s, m);
+  else dft2<PK>(s, m);
+  dft2<PK>(p, q);
+  q = cmul_negi(q);
+  if constexpr (O8) {
+    bf8<PK>(s, p);
+    bf8<PK>(m, q);
+  } else {
+    dft2<PK>(s, p);
+    dft2<PK>(m, q);
+  }
+  a0 = s;
+  a1 = m;
+  a2 = p;
+  a3 = q;
+}
+
 template <int R, bool PK = false>
 __device__ __forceinline__ void dft(float2 (&x)[R]) {
   if constexpr (R == 1) {
@@ -199,26 +250,34 @@ __device__ __forceinline__ void dft(float2 (&x)[R]) {
     // 2 x 4: E = DFT4(even), O = DFT4(odd) * W8^k
     dft4<PK>(x[0], x[2], x[4], x[6]);
     dft4<PK>(x[1], x[3], x[5], x[7]);
-    x[3] = w16<2>(x[3]);
-    x[5] = w16<4>(x[5]);
-    x[7] = w16<6>(x[7]);
+    dft2<PK>(x[0], x[1]);
+    x[3] = w8s<1>(x[3]);
+    bf8<PK>(x[2], x[3]);
+    x[5] = cmul_negi(x[5]);
+    dft2<PK>(x[4], x[5]);
+    x[7] = w8s<3>(x[7]);
+    bf8<PK>(x[6], x[7]);
     float2 y[8];
-    y[0] = badd<PK>(x[0], x[1]); y[4] = bsub<PK>(x[0], x[1]);
-    y[1] = badd<PK>(x[2], x[3]); y[5] = bsub<PK>(x[2], x[3]);
-    y[2] = badd<PK>(x[4], x[5]); y[6] = bsub<PK>(x[4], x[5]);
-    y[3] = badd<PK>(x[6], x[7]); y[7] = bsub<PK>(x[6], x[7]);
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      y[i] = x[2 * i];
+      y[i + 4] = x[2 * i + 1];
+    }
 #pragma unroll
     for (int i = 0; i < 8; i++) x[i] = y[i];
   } else if constexpr (R == 16) {
     // n = n1 + 4 n2, k = k2 + 4 k1
 #pragma unroll
     for (int n1 = 0; n1 < 4; n1++) dft4<PK>(x[n1], x[n1 + 4], x[n1 + 8], x[n1 + 12]);
-    // now x[n1 + 4 k2] = Y[n1][k2]; twiddle W16^{n1 k2}
-    x[5] = w16<1>(x[5]);  x[9] = w16<2>(x[9]);   x[13] = w16<3>(x[13]);
-    x[6] = w16<2>(x[6]);  x[10] = w16<4>(x[10]); x[14] = w16<6>(x[14]);
-    x[7] = w16<3>(x[7]);  x[11] = w16<6>(x[11]); x[15] = w16<9>(x[15]);
-#pragma unroll
-    for (int k2 = 0; k2 < 4; k2++) dft4<PK>(x[4 * k2], x[4 * k2 + 1], x[4 * k2 + 2], x[4 * k2 + 3]);
+    // now x[n1 + 4 k2] = Y[n1][k2]; twiddle W16^{n1 k2} and DFT-4 over n1,
+    // W8's factor in the butterflies' multiply-adds
+    dft4<PK>(x[0], x[1], x[2], x[3]);
+    x[5] = w16<1>(x[5]);   x[6] = w8s<1>(x[6]);           x[7] = w16<3>(x[7]);
+    dft4_8<PK, true, false>(x[4], x[5], x[6], x[7]);
+    x[9] = w8s<1>(x[9]);   x[10] = cmul_negi(x[10]);      x[11] = w8s<3>(x[11]);
+    dft4_8<PK, false, true>(x[8], x[9], x[10], x[11]);
+    x[13] = w16<3>(x[13]); x[14] = w8s<3>(x[14]);         x[15] = w16<9>(x[15]);
+    dft4_8<PK, true, false>(x[12], x[13], x[14], x[15]);
     // now x[4 k2 + k1] = X[k2 + 4 k1]: transpose the 4x4 index
     float2 y[16];
 #pragma unroll

@@ -74,86 +74,30 @@ __device__ __forceinline__ float2 w32(float2 a) {
   constexpr float cs[9] = {1.f, 0.98078528040323044f, AFFT_C8, 0.83146961230254524f, AFFT_R2, 0.55557023301960218f,
                            AFFT_S8, 0.19509032201612825f, 0.f};
   static_assert(K <= 21, "n1 < 4, k2 < 8");
-  if constexpr (K % 4 == 0 && K <= 12) return w16<K / 2>(a);
+  static_assert(K != 4 && K != 12, "these go by w8s");
+  if constexpr (K % 8 == 0 && K < 16) return w16<K / 2>(a);
   else {
     constexpr float x = K < 8 ? cs[K] : K < 16 ? -cs[16 - K] : -cs[K - 16];
     constexpr float y = K < 8 ? -cs[8 - K] : K < 16 ? -cs[K - 8] : cs[24 - K];
-    // (of each component's two products the one by the smaller factor is
-    // rounded by itself)
-    if constexpr (x * x >= y * y) return make_float2(fmaf(a.x, x, -a.y * y), fmaf(a.y, x, a.x * y));
-    else return make_float2(fmaf(-a.y, y, a.x * x), fmaf(a.x, y, a.y * x));
+    return cmulc<(x * x >= y * y)>(a, x, y);
   }
-}
-
-// sqrt(2) W8^K a, K = 1 or 3
-template <int K>
-__device__ __forceinline__ float2 w8s(float2 a) {
-  static_assert(K == 1 || K == 3, "the other powers are 1 and -i");
-  return K == 1 ? make_float2(a.x + a.y, a.y - a.x) : make_float2(a.y - a.x, -a.x - a.y);
-}
-
-// (a, b) = (a + sqrt(1/2) b, a - sqrt(1/2) b): W8's factor in the butterfly's
-// own multiply-add
-template <bool PK>
-__device__ __forceinline__ void bf8(float2& a, float2& b) {
-  const float2 t = a;
-  if constexpr (PK) {
-    a = __ffma2_rn(make_float2(AFFT_R2, AFFT_R2), b, t);
-    b = __ffma2_rn(make_float2(-AFFT_R2, -AFFT_R2), b, t);
-  } else {
-    a = make_float2(fmaf(AFFT_R2, b.x, t.x), fmaf(AFFT_R2, b.y, t.y));
-    b = make_float2(fmaf(-AFFT_R2, b.x, t.x), fmaf(-AFFT_R2, b.y, t.y));
-  }
-}
-
-// DFT-8, natural order in and out, as dft<8> with bf8
-template <bool PK>
-__device__ __forceinline__ void dft8f(float2 (&x)[8]) {
-  dft4<PK>(x[0], x[2], x[4], x[6]);
-  dft4<PK>(x[1], x[3], x[5], x[7]);
-  dft2<PK>(x[0], x[1]);
-  x[3] = w8s<1>(x[3]);
-  bf8<PK>(x[2], x[3]);
-  x[5] = cmul_negi(x[5]);
-  dft2<PK>(x[4], x[5]);
-  x[7] = w8s<3>(x[7]);
-  bf8<PK>(x[6], x[7]);
-  const float2 y1 = x[2], y2 = x[4], y3 = x[6], y4 = x[1], y5 = x[3], y6 = x[5];
-  x[1] = y1; x[2] = y2; x[3] = y3; x[4] = y4; x[5] = y5; x[6] = y6;
 }
 
 // The DFT-32's second half for one k2: twiddles W32^(n1 k2) and a DFT-4 over n1
 template <bool PK, int K2>
 __device__ __forceinline__ void dft32_col(float2 (&x)[32], const float2 (&a)[4][8]) {
   if constexpr (K2 < 8) {
-    float2 s = a[0][K2], m, p, q;
-    if constexpr (K2 == 2 || K2 == 6) {
-      m = w8s<K2 / 2>(a[2][K2]);
-      bf8<PK>(s, m);
-    } else {
-      m = w32<2 * K2>(a[2][K2]);
-      dft2<PK>(s, m);
-    }
+    x[K2] = a[0][K2];
     if constexpr (K2 == 4) {
-      p = w8s<1>(a[1][K2]);
-      q = w8s<3>(a[3][K2]);
+      x[K2 + 8] = w8s<1>(a[1][K2]);
+      x[K2 + 24] = w8s<3>(a[3][K2]);
     } else {
-      p = w32<K2>(a[1][K2]);
-      q = w32<3 * K2>(a[3][K2]);
+      x[K2 + 8] = w32<K2>(a[1][K2]);
+      x[K2 + 24] = w32<3 * K2>(a[3][K2]);
     }
-    dft2<PK>(p, q);
-    q = cmul_negi(q);
-    if constexpr (K2 == 4) {
-      bf8<PK>(s, p);
-      bf8<PK>(m, q);
-    } else {
-      dft2<PK>(s, p);
-      dft2<PK>(m, q);
-    }
-    x[K2] = s;
-    x[K2 + 8] = m;
-    x[K2 + 16] = p;
-    x[K2 + 24] = q;
+    if constexpr (K2 == 2 || K2 == 6) x[K2 + 16] = w8s<K2 / 2>(a[2][K2]);
+    else x[K2 + 16] = w32<2 * K2>(a[2][K2]);
+    dft4_8<PK, K2 == 2 || K2 == 6, K2 == 4>(x[K2], x[K2 + 8], x[K2 + 16], x[K2 + 24]);
     dft32_col<PK, K2 + 1>(x, a);
   }
 }
@@ -169,7 +113,7 @@ __device__ __forceinline__ void dft32(float2 (&x)[32]) {
 #pragma unroll
   for (int i = 0; i < 32; i++) a[i & 3][i >> 2] = x[i];
 #pragma unroll
-  for (int n1 = 0; n1 < 4; n1++) dft8f<PK>(a[n1]);
+  for (int n1 = 0; n1 < 4; n1++) dft<8, PK>(a[n1]);
   dft32_col<PK, 0>(x, a);
 }
 
