@@ -46,6 +46,8 @@ struct LineKernel {
   LineKernelPairedFn paired_tma = nullptr;  // the paired R2C pass over input pairs with TMA-loaded tiles
                                             // (line_fft_paired_tma), or null
   size_t paired_smem = 0;                   // its dynamic shared memory
+  int hilo = 0;                      // every form of the pass takes the four-step twiddle as the hi/lo pair too
+                                     // (axes without a matrix table); else the matrix alone
   int plane_log1 = 0;                // plane kernels (plane_fft): log2 of the rows per plane (the column
                                      // axis); logl is then log2 of the row length; 0 for line kernels
 };
@@ -188,6 +190,7 @@ LineKernel make_line_kernel() {
   k.halves = KIND == LK_R2C_HALF ? 2 : 1;
   k.stage_logl = LOGL + (Sc::E == 32 ? kWideTable : 0);
   k.tstore = TSTORE;
+  k.hilo = KIND == LK_C2R_PAIRED || hilo_twiddle<LOGL, TSTORE, false, UNIT>();
   k.lines_per_cta = C;
   k.threads = Sc::T * C;
   k.smem = (size_t)SmemOf<LOGL, C, COLS, KIND, TSTORE, TC>::FLOAT2S * sizeof(float2);
@@ -208,6 +211,7 @@ LineKernel make_tma_kernel() {
   static_assert(C * sizeof(float) % 16 == 0, "tile columns span whole 16-byte units");
   LineKernel k = make_line_kernel<LOGL, true, KIND, TSTORE, false, UNIT, C>();
   k.tma = &line_fft_tma<LOGL, C, KIND, TSTORE, UNIT>;
+  k.hilo = hilo_twiddle<LOGL, TSTORE, true, UNIT>();
   k.grouped_tma = &line_fft_grouped<LOGL, C, true, KIND, TSTORE, false, UNIT, true>;
   if constexpr (!TSTORE && UNIT == 0 &&
                 ((KIND == LK_C2C &&
@@ -260,6 +264,7 @@ LineKernel make_pipe_kernel() {
   constexpr int C = LOGL == 11 ? AFFT_PIPE_C : 8;
   LineKernel k = make_tma_kernel<LOGL, KIND, C, TSTORE>();
   k.pipe = &line_fft_pipe<LOGL, C, KIND, TSTORE>;
+  k.hilo = 0;
   k.grouped_pipe = TSTORE ? nullptr : &line_fft_pipe_grouped<LOGL, C, KIND>;
   static_assert(LOGL == 11 || LOGL == 10, "the pipelined kernels are built for 1024- and 2048-point lines");
   k.pipe_smem = ((size_t)2 * (1 << LOGL) + pipe_rows<LOGL>()) * C * sizeof(float);   // raw tile + exchange rows

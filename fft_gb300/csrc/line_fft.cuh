@@ -500,7 +500,8 @@ __device__ __forceinline__ void run_stages(float2 (&v)[Sched<LOGL>::E], int t, i
   }
 }
 
-// t2 < 2^11 and k < 2^11, so t2 * k fits 32 bits; L is the line length.
+// t2 k < L times the other factor of the axis = N <= 2^30 (the longest axis),
+// so it fits 32 bits; L is the line length.
 // FULL: read the matrix table tw_full, else the hi/lo pair.
 template <int L, bool FULL>
 __device__ __forceinline__ float2 fourstep_twiddle(const LineParams& p, long long q, int k) {
@@ -513,6 +514,17 @@ __device__ __forceinline__ float2 fourstep_twiddle(const LineParams& p, long lon
     float2 b = ldg2(p.tw_lo + (m & ((1 << p.tw_lo_bits) - 1)));
     return cmul(a, b);
   }
+}
+
+// Whether a complex cols kernel has code for the hi/lo pair.  Axes of up to
+// 2^22 points have the matrix table; longer ones go without, and of their
+// passes only the first, 256 points with the transposing store, multiplies by
+// W_N (its rest is a four-step of 2^22 points at most): that kernel has both
+// in every form.  The no-allocation entry point has the pair alone at every
+// length, and launches the split LSU kernels.
+template <int LOGL, bool TSTORE, bool TMA, int UNIT>
+constexpr bool hilo_twiddle() {
+  return (TSTORE && LOGL == 8) || (!TMA && UNIT == 0);
 }
 
 // ---------------------------------------------------------------------------
@@ -1326,9 +1338,8 @@ __device__ __forceinline__ void line_fft_body(const LineParams& p, long long cta
         const long long base = line_off(p.out, q2);
         const bool inv = p.inverse;
         // one branch-free loop per case, so the twiddle loads issue together
-        // (every transposing pass has the twiddle; the hi/lo pair is the
-        // no-allocation entry point's, which launches the split LSU kernels)
-        constexpr bool HILO = !TMA && UNIT == 0;
+        // (every transposing pass has the twiddle)
+        constexpr bool HILO = hilo_twiddle<LOGL, true, TMA, UNIT>();
         // the four-step passes store with unit element stride: compile-time
         // offsets from one pointer per array; other strides as the loads
         const long long S = (long long)T * p.out.es;
@@ -1355,11 +1366,16 @@ __device__ __forceinline__ void line_fft_body(const LineParams& p, long long cta
           float* pz = p.out.re + base + 2LL * t2;
           if (p.out.es == 2 && !(reinterpret_cast<uintptr_t>(pz) & 7)) {
             float2* pp = reinterpret_cast<float2*>(pz);
+            auto emit2 = [&](auto full) {
 #pragma unroll
-            for (int e = 0; e < E; e++) {
-              const float2 x = cmul(sm.get(c2, t2 + T * e), fourstep_twiddle<L, true>(p, q2, t2 + T * e));
-              pp[T * e] = inv ? cswap(x) : x;
-            }
+              for (int e = 0; e < E; e++) {
+                const float2 x =
+                    cmul(sm.get(c2, t2 + T * e), fourstep_twiddle<L, decltype(full)::value>(p, q2, t2 + T * e));
+                pp[T * e] = inv ? cswap(x) : x;
+              }
+            };
+            if (!HILO || p.tw_full) emit2(std::true_type{});
+            else if constexpr (HILO) emit2(std::false_type{});
             stored = true;
           }
         }
@@ -1373,7 +1389,7 @@ __device__ __forceinline__ void line_fft_body(const LineParams& p, long long cta
     } else {
       // four-step twiddles only occur in cols passes
       if constexpr (COLS) {
-        constexpr bool HILO = !TMA && UNIT == 0;   // as above
+        constexpr bool HILO = hilo_twiddle<LOGL, false, TMA, UNIT>();
         if (p.tw_n && (!HILO || p.tw_full)) {
 #pragma unroll
           for (int e = 0; e < E; e++) v[e] = cmul(v[e], fourstep_twiddle<L, true>(p, q, t + T * e));

@@ -558,6 +558,10 @@ struct Builder {
       op.k = ka;
       if (!AFFT_COLS_TMA || tune.cols_lsu) op.k.tma = nullptr, op.k.grouped_tma = nullptr, op.k.tma_bulk = nullptr;
     }
+    if (tw_n > kFullTableMax && !f64 && !op.k.hilo) {
+      fail("no kernel for this pass of an axis without a matrix twiddle table");
+      return;
+    }
     op.in = in;
     op.out = out;
     op.p.nlines = nlines;
@@ -1057,11 +1061,12 @@ std::string describe_plan(const Plan& P) {
                "{\"type\":\"line\",\"logl\":%d,\"cols\":%d,\"lk\":%d,\"tstore\":%d,\"tc\":%d,\"C\":%d,"
                "\"halves\":%d,\"unit\":%d,\"tma\":%d,\"tma_store\":%d,\"pipe\":%d,\"plane\":%d,"
                "\"threads\":%d,\"smem\":%zu,\"grid\":%lld,\"nlines\":%lld,\"inverse\":%d,"
-               "\"tw_n\":%lld,\"tw_qmask\":%lld,\"tw_qshift\":%d,\"real_L\":%lld,\"pcols\":%lld,",
+               "\"tw_n\":%lld,\"tw_qmask\":%lld,\"tw_qshift\":%d,\"hilo\":%d,\"real_L\":%lld,\"pcols\":%lld,",
                op.k.logl, op.k.cols, op.k.kind, op.k.tstore, op.k.tc, op.k.lines_per_cta, op.k.halves, op.k.unit,
                op.k.tma != nullptr, op.k.tma_bulk != nullptr, op.k.pipe != nullptr, op.k.plane_log1, op.threads,
                op.smem,
-               op.grid, op.p.nlines, op.p.inverse, op.p.tw_n, op.p.tw_qmask, op.p.tw_qshift, op.real_L, op.p.pcols);
+               op.grid, op.p.nlines, op.p.inverse, op.p.tw_n, op.p.tw_qmask, op.p.tw_qshift, op.k.hilo,
+               op.real_L, op.p.pcols);
     } else if (op.type == OP_REAL) {
       snprintf(buf, sizeof buf,
                "{\"type\":\"real\",\"threads\":%d,\"grid\":%lld,\"nlines\":%lld,\"L\":%lld,"
@@ -1205,7 +1210,7 @@ bool tma_paired(const LineParams& p, const LineKernel& k, PairedTma* pt) {
 bool op_tables_ok(const Op& op) {
   if (op.type != OP_LINE) return op.type != OP_REAL || op.rp.rtw;
   return op.p.tw && (op.k.kind == LK_C2C || op.p.rtw) &&
-         (!op.p.tw_n || op.p.tw_full || (op.p.tw_hi && op.p.tw_lo)) && (!op.k.tc || op.p.tc_b) &&
+         (!op.p.tw_n || op.p.tw_full || (op.k.hilo && op.p.tw_hi && op.p.tw_lo)) && (!op.k.tc || op.p.tc_b) &&
          (!op.k.plane_log1 || op.p.tw2);
 }
 

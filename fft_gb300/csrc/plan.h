@@ -151,10 +151,10 @@ const float2* real_twiddles(long long L);         // W_{2L}^k, k < L
 void fourstep_tables(long long N, const float2** hi, const float2** lo, int* lo_bits);
 // The four-step twiddle as one matrix, W_N^{t2 k} at [t2 * L1 + k], for
 // N <= kFullTableMax (nullptr above): one coalesced load per element.  It
-// covers every four-step axis a plan builds (up to 2^22 points: 32 MB), so
-// each plan's four-step twiddle is computed in FP64 and rounded once; the
-// hi/lo product form remains for the no-allocation entry point's fixed
-// arrays.
+// covers every four-step axis of up to 2^22 points (32 MB), whose twiddle is
+// then computed in FP64 and rounded once; the hi/lo product form remains for
+// longer axes (the first of their three passes) and for the no-allocation
+// entry point's fixed arrays.  LineKernel::hilo says which kernels take it.
 #ifndef AFFT_FULL_TABLE_LOG
 #define AFFT_FULL_TABLE_LOG 22
 #endif
