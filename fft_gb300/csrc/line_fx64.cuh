@@ -9,16 +9,22 @@
 // are rounded to double once at the end.
 //
 // Precision.  A line's values are held with the largest one's top bit at
-// bit 57 to 60, so the unit is at most 2^-57 of the line's largest value,
+// bit 59 or 60 (57 to 60 before the first stage, by what it may grow), so the
+// unit is at most 2^-59 of the line's largest value (2^-57),
 // against 2^-53 relative roundoff per FP64 operation.  Between two stages the
-// line is shifted (by the OR of all magnitudes, so no headroom is spent that
+// line is shifted (by the largest magnitude, so no headroom is spent that
 // the data do not need) to keep it that way.  Products by a twiddle use its
 // 62-bit fixed-point value; the low x low partial product, at most a quarter
 // unit, is dropped.  The error is therefore relative to the line's norm, as
-// that of the FP64 butterflies is, and smaller: against extended-precision
-// FFTs of normal data 0.86e-16 at 4096 points (FP64: 2.4e-16), 1.2e-16 at
-// 2^17 (2.8e-16); with one value 1e5 times the others 1.4 to 2.0e-16 (2.2 to
-// 2.8e-16).
+// that of the FP64 butterflies is, and smaller.  Relative L2 error in 1e-16
+// against extended-precision FFTs (FP64 butterflies in brackets): 4096 points
+// normal 0.9 (2.3), uniform(0,1) 0.7 (2.1), the same with one 1e5 1.0 (2.2);
+// real inverses of the spectra of 8192 and 16384 reals 10 + normal 1.1 and
+// 1.6 (1.9).
+// What it does not have is the luck of values that FP64 never adds to larger
+// ones: a value 2^-k of its line's largest is held in 60 - k bits, so of a
+// line whose large values cancel exactly (even elements 1, odd ones 1e-12),
+// bins that only the small ones reach carry the line's error, not their own.
 //
 // Range.  Lines with a non-finite value, one above 2^977, or nonzero data
 // below 2^-823 are left to the FP64 body of the same kernel (the whole CTA
@@ -26,7 +32,7 @@
 //
 // Bounds, in bits (component magnitudes; |z| is the complex magnitude): first
 // stage's output |z| < 2^62.5, every intermediate < 2^63; before a twiddle
-// product the line's top bit is bit 57 to 60 (59 before the last stage of a
+// product the line's top bit is bit 59 or 60 (59 before the last stage of a
 // real forward pass; components < 2^61, |z| < 2^61.5); the product is scaled
 // by 1/4: |z| < 2^59.5, and < 2^62.5 after the next radix-8 stage.
 #pragma once
@@ -49,9 +55,9 @@ constexpr int fx_top() {
   using Sc = Sched64<LOGL>;
   return Sc::FIRST == 2 ? 60 : Sc::FIRST == 4 ? 59 : Sc::NSTAGES > 1 ? 58 : 57;
 }
-constexpr int FX_TOP_TW = 59;     // the same where a twiddle product follows, when shifted there
-constexpr int FX_TOP_MIN = 57, FX_TOP_MAX = 60;   // and where it is left as it is (59 before the last stage of
-                                                  // a pass that adds its output in pairs, the real forward)
+constexpr int FX_TOP_MIN = 59, FX_TOP_MAX = 60;   // the same where a twiddle product follows; MIN before the last
+                                                  // stage of a pass that adds its output in pairs, the real forward
+constexpr int FX_TOP_C2R = 59;    // and of a real inverse's bins, before its pre-pass (which may grow them fourfold)
 constexpr int FX_EXP_MIN = 200;   // biased exponents the fixed-point form takes: below, subnormal results are
 constexpr int FX_EXP_MAX = 2000;  // possible; above, overflow (14 bits of growth) and non-finite values
 
@@ -60,9 +66,15 @@ __device__ __forceinline__ int fx_lo(fx a) { return (int)a; }
 // a = fx_s1(a) * 2^32 + (signed) fx_lo(a)
 __device__ __forceinline__ int fx_s1(fx a) { return fx_hi(a) + (int)((unsigned)fx_lo(a) >> 31); }
 __device__ __forceinline__ fx mw(int a, int b) { return (fx)a * (fx)b; }
-// a / 2^n to nearest, ties away from zero: a mean of half a tie would add up
-// over a line to an error in bin 0
+// a / 2^n to nearest, ties away from zero, or to even: a mean of half a tie
+// would add up over a line to an error in bin 0.  Away where it is input 0 of
+// a butterfly: of the products by 1 beside it those of inputs 1, 2 and 5 round
+// ties away from zero and the others towards it (split62 in plan.cu), so that
+// on data of one sign the eight have no mean, nor one large harmonic (the
+// sign's DFT is 0, 2.8, 4, 2.8, 0; alternating signs put 1.3e-15 of 16384
+// positive reals with a spike into one bin, these 0.9e-15, FP64 0.8e-15).
 __device__ __forceinline__ fx fx_sar(fx a, int n) { return (a + (1LL << (n - 1)) + (a >> 63)) >> n; }
+__device__ __forceinline__ fx fx_sar_even(fx a, int n) { return (a + ((1LL << (n - 1)) - 1) + ((a >> n) & 1)) >> n; }
 
 __device__ __forceinline__ fxc cadd(fxc a, fxc b) { return {a.x + b.x, a.y + b.y}; }
 __device__ __forceinline__ fxc csub(fxc a, fxc b) { return {a.x - b.x, a.y - b.y}; }
@@ -123,17 +135,18 @@ __device__ __forceinline__ void fx_dft(fxc (&x)[R]) {
 
 __device__ __forceinline__ int d_hi(double v) { return __double2hiint(v); }
 
-// The double's value in units of 2^(emax - 1023 - TOP), rounded towards
-// zero; emax: the line's largest biased exponent field
+// The double's value in units of 2^(emax - 1023 - TOP), rounded to nearest
+// (half a unit lost by each small value would add up in bin 0 of a positive
+// line); emax: the line's largest biased exponent field
 template <int TOP>
 __device__ __forceinline__ fx fx_from(double v, int emax) {
   const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
   const unsigned m = (hi & 0xfffffu) | 0x100000u;
-  const int sh = (int)(((unsigned)(emax + 63 - TOP) << 20) + 0xfffffu - (hi & 0x7fffffffu)) >> 20;
+  const int sh = (int)(((unsigned)(emax + 62 - TOP) << 20) + 0xfffffu - (hi & 0x7fffffffu)) >> 20;
   unsigned long long u = ((unsigned long long)__funnelshift_l(lo, m, 11) << 32) | (lo << 11);
   asm("shr.u64 %0, %0, %1;" : "+l"(u) : "r"(sh));   // PTX clamps the amount: zeros and tiny values give 0
   const fx s = (fx)((int)hi >> 31);
-  return ((fx)u ^ s) - s;
+  return (((fx)u ^ s) + 1) >> 1;   // u: twice the magnitude; -u = ~u + 1
 }
 
 // a * 2^sc as the nearest double (sc << 20 given; no subnormal or overflowing result in the range this form takes)
@@ -226,21 +239,25 @@ struct FxSmem {
   }
 };
 
-// Shift a line whose FxMag word is m to top bit FX_TOP_TW, the exponent
-// following, unless it is near enough (normal data stays within the range by
-// itself: a radix-8 stage grows it by 1.5 bits, the product takes 2)
+// bit of the largest magnitude of a line whose FxMag word is m
+__device__ __forceinline__ int fx_top_of(int m) { return 62 - __clz(m); }
+
+// Shift a line whose FxMag word is m to top bit MAX, the exponent following,
+// unless it is near enough (normal data mostly stays within the range by
+// itself: a radix-8 stage grows it by 1.5 bits, the product takes 2; a line
+// that one value dominates does not grow)
 template <int MAX, int E>
 __device__ __forceinline__ void fx_level(fxc (&v)[E], int m, int& sc) {
-  const int top = 62 - __clz(m);   // bit of the line's largest magnitude
+  const int top = fx_top_of(m);
   if (top >= FX_TOP_MIN && top <= MAX) return;
-  const int n = FX_TOP_TW - top;
+  const int n = MAX - top;
   sc -= n;
   if (n > 0) {
 #pragma unroll
     for (int e = 0; e < E; e++) v[e] = {v[e].x << n, v[e].y << n};
   } else {
 #pragma unroll
-    for (int e = 0; e < E; e++) v[e] = {fx_sar(v[e].x, -n), fx_sar(v[e].y, -n)};
+    for (int e = 0; e < E; e++) v[e] = {fx_sar_even(v[e].x, -n), fx_sar_even(v[e].y, -n)};
   }
 }
 
@@ -289,7 +306,7 @@ __device__ __forceinline__ void fx_stages(fxc (&v)[Sched64<LOGL>::E], int t, int
       for (int e = 0; e < E; e++) v[e] = sm.get(c, t + T * e);
       if constexpr (!Ln::REG) mag = slots[(S + 1) * C + c];
       if constexpr (S + 1 < Sc::NSTAGES - 1) line_sync<WARP_ONLY>();   // every gather is done before the next scatter
-      fx_level<PAIRS && S + 1 == Sc::NSTAGES - 1 ? FX_TOP_TW : FX_TOP_MAX>(v, mag, sc);
+      fx_level<PAIRS && S + 1 == Sc::NSTAGES - 1 ? FX_TOP_MIN : FX_TOP_MAX>(v, mag, sc);
       fx_stages<LOGL, C, COLS, WARP_ONLY, PAIRS, S + 1>(v, t, c, tw, sm, slots, sc);
     }
   }
@@ -309,7 +326,9 @@ __device__ __forceinline__ void line_fx64_body(const LineParams& p, long long ct
   constexpr bool WARP_ONLY = (!COLS && T <= 32) || (T * C <= 32);
   using Ln = FxLine<T, C, COLS>;
   extern __shared__ __align__(1024) double2 smem64[];
-  __shared__ int slots[(Sc::NSTAGES + 1) * C];   // row 0: largest exponents (then the lines' scales), rows 1..: ORs
+  // row 0: largest exponents (then the lines' scales), rows 1..: ORs of the magnitudes after each stage but the
+  // last, whose row has those of the real inverse's pre-pass
+  __shared__ int slots[(Sc::NSTAGES + 1) * C];
   FxSmem<L, C, COLS> sm{{smem64}};
   const int4* tw = reinterpret_cast<const int4*>(p.tw);
   const int4* rtw = reinterpret_cast<const int4*>(p.rtw);
@@ -373,14 +392,20 @@ __device__ __forceinline__ void line_fx64_body(const LineParams& p, long long ct
 
   fxc v[E];
   if constexpr (KIND == LK_C2R) {
-    // Z'[i] = a - i*b as line_fft64_body, |Z'| up to four times the bins: two
-    // bits lower.  A pair of bins at a time, i from the lower half of the line
+    // Z'[i] = a - i*b as line_fft64_body, |Z'| up to four times the bins (<
+    // 2^62.5), so the line is shifted to what the first stage takes only then,
+    // when its magnitudes are known: where bin 0 dominates (data with a mean)
+    // nothing grows, and two bits fewer from the start would cost it twice
+    // the error of FP64 (8192 reals 10 + normal 9.0e-16, now 1.1e-16).
+    // A pair of bins at a time, i from the lower half of the line
     // and L - i, whose a and b are the conjugates: Z'[L-i] = conj(a + i b).
     // The upper half's bins go through shared memory and its Z' come back the
     // same way (element L - i is this thread's alone in between).
-    sc += 2;
+    constexpr int IN = FX_TOP_C2R;
+    sc += TOP - IN;
+    FxMag<!(COLS && LOGL == 8)> seen;
 #pragma unroll
-    for (int e = 0; e < E; e++) v[e] = {fx_from<TOP - 2>(d[e].x, emax), fx_from<TOP - 2>(d[e].y, emax)};
+    for (int e = 0; e < E; e++) v[e] = {fx_from<IN>(d[e].x, emax), fx_from<IN>(d[e].y, emax)};
 #pragma unroll
     for (int e = E / 2; e < E; e++) sm.put(c, t + T * e, v[e]);
     line_sync<WARP_ONLY>();
@@ -389,7 +414,7 @@ __device__ __forceinline__ void line_fx64_body(const LineParams& p, long long ct
       const int i = t + T * e;
       fxc z, zl;
       if (i == 0) {   // from the real parts of X[0] and X[L]; Z'[L/2] = 2 conj(X[L/2])
-        const fx r1 = fx_from<TOP - 2>(dL, emax);
+        const fx r1 = fx_from<IN>(dL, emax);
         z = {v[0].x + r1, v[0].x - r1};
         zl = {2 * v[E / 2].x, -2 * v[E / 2].y};
       } else {
@@ -403,13 +428,25 @@ __device__ __forceinline__ void line_fx64_body(const LineParams& p, long long ct
         zl = cadd_i(a, b);
         zl.y = -zl.y;
       }
+      seen.add(z);
+      seen.add(zl);
       v[e] = {z.y, z.x};
       sm.put(c, i == 0 ? L / 2 : L - i, {zl.y, zl.x});
     }
+    int mag = seen.word();
+    if constexpr (Ln::REG) mag = Ln::in_regs_or(mag);
+    else Ln::publish_or(mag, slots + Sc::NSTAGES * C, c);
     line_sync<WARP_ONLY>();
 #pragma unroll
     for (int e = E / 2; e < E; e++) v[e] = sm.get(c, t + T * e);
+    if constexpr (!Ln::REG) mag = slots[Sc::NSTAGES * C + c];
     line_sync<WARP_ONLY>();   // before the stages write the buffer
+    const int n = fx_top_of(mag) - TOP;
+    if (n > 0) {
+      sc += n;
+#pragma unroll
+      for (int e = 0; e < E; e++) v[e] = {fx_sar_even(v[e].x, n), fx_sar_even(v[e].y, n)};
+    }
   } else {
 #pragma unroll
     for (int e = 0; e < E; e++) {

@@ -292,21 +292,21 @@ const float2* fourstep_full_table(long long N, long long L2) {
 // FP64 tables: the same roots in 62-bit fixed point, each component as high *
 // 2^32 + low with a signed low word (never -2^31: the kernels negate it).
 // The FP64 value's own error (2^-54) is the larger one.
-static void split62(double v, int* hi, int* lo) {
+static void split62(double v, bool away, int* hi, int* lo) {
   const long long w = std::llrint(std::ldexp(v, 62));
   *hi = (int)((w + (1LL << 31)) >> 32);
   *lo = (int)(w - (long long)*hi * (1LL << 32));
   if (*lo == INT_MIN) *lo += 1;
-  // +-1 exactly: one unit (2^-62) nearer to zero, so that the products' exact
-  // quarters round their ties by the sign of the data and leave no mean
-  if (*lo == 0 && *hi != 0) *lo = *hi > 0 ? -1 : 1;
+  // +-1 exactly: one unit (2^-62) nearer to zero or away from it, so that the
+  // products' exact quarters round their ties by the sign of the data
+  if (*lo == 0 && *hi != 0) *lo = (*hi > 0) == away ? 1 : -1;
 }
-static int4 root_d(long long m, long long N) {
+static int4 root_d(long long m, long long N, bool away = false) {
   double c, s;
   unit_root(m, N, &c, &s);
   int4 w;
-  split62(c, &w.x, &w.y);
-  split62(s, &w.z, &w.w);
+  split62(c, away, &w.x, &w.y);
+  split62(s, away, &w.z, &w.w);
   return w;
 }
 
@@ -319,7 +319,8 @@ static std::vector<int4> stage_table64() {
     if (ns == 1) continue;
     int off = S::twoff(s);
     for (int r = 1; r < R; r++)
-      for (int k = 0; k < ns; k++) t[off + (r - 1) * ns + k] = root_d((long long)r * k, (long long)ns * R);
+      for (int k = 0; k < ns; k++)   // (away from zero for r = 1, 2, 5: fx_sar in line_fx64.cuh)
+        t[off + (r - 1) * ns + k] = root_d((long long)r * k, (long long)ns * R, (0x26 >> r) & 1);
   }
   return t;
 }

@@ -118,7 +118,8 @@ AFFT_GB300_API size_t afft_32_align_size(size_t sz);
 /* Replaces fft.h:48-80 (FP64): the same transforms, layouts, errors and
  * pointer rules on double arrays, to FP64 accuracy: lines are transformed in
  * 64-bit block fixed point (one exponent per line, relative L2 error 1e-16 to
- * 3e-16), lines that do not fit it on the FP64 pipe.  A plan made by an
+ * 3e-16: an error relative to the line's norm, so values 2^-k of its largest
+ * keep 60 - k bits), lines that do not fit it on the FP64 pipe.  A plan made by an
  * afft_64_*_create (or a batched plan with AFFT_GB300_FORM_F64) runs only
  * through the afft_64_* transforms, an FP32 plan only through the afft_32_*
  * ones; a mismatch sets AFFT_GB300_EINVAL and launches nothing. */
