@@ -207,9 +207,10 @@ __device__ __forceinline__ void std_(float* base, long long off, double v) {
 // the pre-pass fused into the loads), with the algebra of afft's real_pass
 // (onedim.hpp:1031-1108, multi.hpp:343-414).  TSTORE (cols c2c): computed
 // with the cols mapping, stored with the rows mapping, the four-step twiddle
-// applied on the way out.
+// applied on the way out.  only: per line of the tile, whether it is loaded and
+// stored (null: all are).
 template <int LOGL, int C, bool COLS, int KIND, bool TSTORE>
-__device__ __forceinline__ void line_fft64_body(const LineParams& p, long long cta) {
+__device__ __forceinline__ void line_fft64_body(const LineParams& p, long long cta, const int* only = nullptr) {
   using Sc = Sched64<LOGL>;
   constexpr int L = Sc::L, E = Sc::E, T = Sc::T;
   constexpr bool WARP_ONLY = (!COLS && T <= 32) || (T * C <= 32);
@@ -222,7 +223,7 @@ __device__ __forceinline__ void line_fft64_body(const LineParams& p, long long c
   const int c = COLS ? (tid % C) : (tid / T);
   const int t = COLS ? (tid / C) : (tid % T);
   const long long q = cta * C + c;
-  const bool active = q < p.nlines;
+  const bool active = q < p.nlines && (!only || only[c]);
 
   double2 v[E];
   if (!active) {
@@ -273,7 +274,7 @@ __device__ __forceinline__ void line_fft64_body(const LineParams& p, long long c
     __syncthreads();
     const int c2 = tid / T, t2 = tid % T;
     const long long q2 = cta * C + c2;
-    if (q2 < p.nlines) {
+    if (q2 < p.nlines && (!only || only[c2])) {
       const long long base = line_off(p.out, q2);
       const int4* twf = reinterpret_cast<const int4*>(p.tw_full);
       const int r2 = (int)((q2 >> p.tw_qshift) & p.tw_qmask);

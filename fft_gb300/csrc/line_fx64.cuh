@@ -27,8 +27,10 @@
 // bins that only the small ones reach carry the line's error, not their own.
 //
 // Range.  Lines with a non-finite value, one above 2^977, or nonzero data
-// below 2^-823 are left to the FP64 body of the same kernel (the whole CTA
-// takes it), so infinities, NaNs, overflow and subnormals behave as there.
+// below 2^-823 throughout are left to the FP64 body of the same kernel, so
+// infinities, NaNs, overflow and subnormals behave as there; the other lines
+// of their tile are not, so no line's result depends on its neighbours.
+// (Zeros come out as +0, whatever the signs of the zeros that went in.)
 //
 // Bounds, in bits (component magnitudes; |z| is the complex magnitude): first
 // stage's output |z| < 2^62.5, every intermediate < 2^63; before a twiddle
@@ -314,8 +316,13 @@ __device__ __forceinline__ void fx_stages(fxc (&v)[Sched64<LOGL>::E], int t, int
 
 // the FP64 body, for the lines the fixed-point form leaves to it
 template <int LOGL, int C, bool COLS, int KIND, bool TSTORE>
-__device__ __noinline__ void line_fft64_general(const LineParams& p, long long cta) {
-  line_fft64_body<LOGL, C, COLS, KIND, TSTORE>(p, cta);
+__device__ __noinline__ void line_fft64_general(const LineParams& p, long long cta, const int* only) {
+  line_fft64_body<LOGL, C, COLS, KIND, TSTORE>(p, cta, only);
+}
+
+// whether a line whose largest high word (sign off) is top goes there; 1: all zeros and subnormals
+__device__ __forceinline__ bool fx_out_of_range(int top) {
+  return (top >> 20) > FX_EXP_MAX || (top > 0 && (top >> 20) < FX_EXP_MIN);
 }
 
 // The kernel body for one CTA (C lines), arguments as line_fft64_body.
@@ -329,6 +336,7 @@ __device__ __forceinline__ void line_fx64_body(const LineParams& p, long long ct
   // row 0: largest exponents (then the lines' scales), rows 1..: ORs of the magnitudes after each stage but the
   // last, whose row has those of the real inverse's pre-pass
   __shared__ int slots[(Sc::NSTAGES + 1) * C];
+  __shared__ int odd_of[C];   // lines left to the FP64 body
   FxSmem<L, C, COLS> sm{{smem64}};
   const int4* tw = reinterpret_cast<const int4*>(p.tw);
   const int4* rtw = reinterpret_cast<const int4*>(p.rtw);
@@ -371,20 +379,18 @@ __device__ __forceinline__ void line_fx64_body(const LineParams& p, long long ct
   int top = KIND == LK_C2R ? d_hi(dL) & 0x7fffffff : 0;
 #pragma unroll
   for (int e = 0; e < E; e++) top = max(top, max(d_hi(d[e].x) & 0x7fffffff, d_hi(d[e].y) & 0x7fffffff));
-  // a nonzero top below 2^FX_EXP_MIN: too small, or another thread holds the line's large values; take no chance
-  bool odd = (top >> 20) > FX_EXP_MAX || (top > 0 && (top >> 20) < FX_EXP_MIN);
   if (top == 0) {   // subnormals too small to show in a high word
     int low = KIND == LK_C2R ? __double2loint(dL) : 0;
 #pragma unroll
     for (int e = 0; e < E; e++) low |= __double2loint(d[e].x) | __double2loint(d[e].y);
-    odd = low != 0;
+    top = low != 0;
   }
+  // a line goes by its largest value; the thread that holds it says so first
+  const bool maybe = fx_out_of_range(top);
   if constexpr (Ln::REG) top = Ln::in_regs_max(top);
   else Ln::publish_max(top, slots, c);
-  if (__syncthreads_or(odd)) {
-    line_fft64_general<LOGL, C, COLS, KIND, TSTORE>(p, cta);
-    return;
-  }
+  const bool rare = __syncthreads_or(maybe);
+  if (rare && t == 0) odd_of[c] = fx_out_of_range(Ln::REG ? top : slots[c]);
   if constexpr (!Ln::REG) top = slots[c];
   constexpr int TOP = fx_top<LOGL>();
   const int emax = max(top >> 20, FX_EXP_MIN);   // (a line of zeros: every element shifts out)
@@ -464,7 +470,7 @@ __device__ __forceinline__ void line_fx64_body(const LineParams& p, long long ct
     __syncthreads();
     const int c2 = tid / T, t2 = tid % T;
     const long long q2 = cta * C + c2;
-    if (q2 < p.nlines) {
+    if (q2 < p.nlines && !(rare && odd_of[c2])) {
       const long long ob = line_off(p.out, q2);
       const int4* twf = reinterpret_cast<const int4*>(p.tw_full);
       const int r2 = (int)((q2 >> p.tw_qshift) & p.tw_qmask);
@@ -486,7 +492,7 @@ __device__ __forceinline__ void line_fx64_body(const LineParams& p, long long ct
 #pragma unroll
     for (int e = E / 2; e < E; e++) sm.put(c, t + T * e, v[e]);
     line_sync<WARP_ONLY>();
-    if (active) {
+    if (active && !(rare && odd_of[c])) {
       const long long ob = line_off(p.out, q);
       const int sc20 = sc * (1 << 20);
       auto emit = [&](int k, fxc x) {
@@ -523,7 +529,7 @@ __device__ __forceinline__ void line_fx64_body(const LineParams& p, long long ct
         sc += 2;
       }
     }
-    if (active) {
+    if (active && !(rare && odd_of[c])) {
       const long long ob = line_off(p.out, q);
       const int sc20 = sc * (1 << 20);
 #pragma unroll
@@ -534,6 +540,9 @@ __device__ __forceinline__ void line_fx64_body(const LineParams& p, long long ct
       }
     }
   }
+  // (after the others' stores, which go to other lines: a call before them
+  // would cost every kernel 100 to 200 bytes of spills)
+  if (rare && __syncthreads_or(odd_of[c])) line_fft64_general<LOGL, C, COLS, KIND, TSTORE>(p, cta, odd_of);
 }
 
 // 1024 resident threads (64 registers each): at the 80 to 120 registers the
