@@ -15,6 +15,7 @@ library cannot be loaded, importing this module raises.
 """
 import ctypes
 import os
+import sys
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libafft_gb300.so")
@@ -134,9 +135,11 @@ def ptr(a):
     f = getattr(a, "data_ptr", None)
     if f is not None:
         return f()
-    f = getattr(a, "__array_interface__", None)   # numpy: a quarter of the time of a.ctypes.data
-    if f is not None:
-        return f["data"][0]
+    numpy = sys.modules.get("numpy")
+    if numpy is not None and type(a) is numpy.ndarray:
+        # a quarter of the time of a.ctypes.data; of arrays alone: others give
+        # bytes here, or the address of a temporary (numpy's scalars)
+        return a.__array_interface__["data"][0]
     if hasattr(a, "ctypes"):
         return a.ctypes.data
     raise TypeError(type(a))
