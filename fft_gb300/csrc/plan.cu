@@ -765,7 +765,7 @@ struct Builder {
       // (FP64: from 2^20 points a line and 2^23 in all, 16 x 2^20 582 -> 468
       // us, 4 x 2^22 796 -> 597, 32 x 2^19 513 -> 582; up to 4 GB of scratch,
       // two passes where the device has not that much left)
-      const bool three = f64 ? tune.passes != 2 && logl >= 20 && pts >= (1LL << 23) && pts <= (1LL << 27)
+      const bool three = f64 ? tune.passes != 2 && logl >= 20 && logl <= 22 && pts >= (1LL << 23) && pts <= (1LL << 27)
                              : (tune.passes == 3 ? logl >= 20 : tune.passes == 2 ? false : logl >= AFFT_THREE_PASS_LOG);
       int l1 = three ? 8 : l1_of(logl), l2 = logl - l1;
       if (l1 > COLS_MAX_LOG || (l2 > COLS_MAX_LOG && !three)) {
