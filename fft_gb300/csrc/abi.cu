@@ -149,23 +149,18 @@ static size_t memsize_impl(int kind, size_t ndim, const size_t* dim, size_t batc
 }
 
 // A plan with its device scratch, so later launches allocate nothing (and can
-// be captured into CUDA graphs).  FP64 axes in three passes take twice the
-// scratch of two: where that much is not free, two passes.
+// be captured into CUDA graphs).
 static std::unique_ptr<Plan> build_with_scratch(int kind, int ndim, const long long* dims, long long batch,
                                                 int format, int form) {
-  Tuning two;
-  two.passes = 2;
-  for (const Tuning* t : {(const Tuning*)nullptr, (const Tuning*)&two}) {
-    auto P = build_plan(kind, ndim, dims, batch, format, false, form, t);
-    if (!P) return nullptr;
-    if (P->scratch_elems == 0 || cudaMalloc(&P->scratch, (size_t)P->scratch_elems * P->esize()) == cudaSuccess)
-      return P;
+  auto P = build_plan(kind, ndim, dims, batch, format, false, form);
+  if (!P) return nullptr;
+  if (P->scratch_elems > 0 && cudaMalloc(&P->scratch, (size_t)P->scratch_elems * P->esize()) != cudaSuccess) {
     cudaGetLastError();
     P->scratch = nullptr;
-    if (!P->f64()) break;
+    set_error(AFFT_GB300_ENOMEM, "scratch allocation failed");
+    return nullptr;
   }
-  set_error(AFFT_GB300_ENOMEM, "scratch allocation failed");
-  return nullptr;
+  return P;
 }
 
 static void* create_impl(int kind, size_t ndim, const size_t* dim, size_t batch, int format, void* mem,

@@ -740,9 +740,10 @@ struct Builder {
 
   // Complex transform along the middle axis of a dense (outer, L, inner)
   // array, from view A to view B (may be the same).  a_bs / b_bs: complex
-  // elements between outer blocks (default L*inner).
+  // elements between outer blocks (default L*inner).  over_a: a strided axis's
+  // first pass may write over A (dense scratch that nothing else reads).
   void axis(long long outer, long long L, long long inner, const View& A, const View& B,
-            bool inverse, long long a_bs = 0, long long b_bs = 0) {
+            bool inverse, long long a_bs = 0, long long b_bs = 0, bool over_a = false) {
     if (!ok) return;
     if (a_bs == 0) a_bs = L * inner;
     if (b_bs == 0) b_bs = L * inner;
@@ -763,9 +764,9 @@ struct Builder {
       // of 1024 / 2048, whose one-CTA-per-SM tiles run at about half the
       // rate per pass
       // (FP64: from 2^20 points a line and 2^23 in all, 16 x 2^20 582 -> 468
-      // us, 4 x 2^22 796 -> 597, 32 x 2^19 513 -> 582; up to 4 GB of scratch,
-      // two passes where the device has not that much left)
-      const bool three = f64 ? tune.passes != 2 && logl >= 20 && logl <= 22 && pts >= (1LL << 23) && pts <= (1LL << 27)
+      // us, 4 x 2^22 796 -> 597, 32 x 2^19 513 -> 582; nothing was timed
+      // beyond 2^27)
+      const bool three = f64 ? logl >= 20 && logl <= 22 && pts >= (1LL << 23) && pts <= (1LL << 27)
                              : (tune.passes == 3 ? logl >= 20 : tune.passes == 2 ? false : logl >= AFFT_THREE_PASS_LOG);
       int l1 = three ? 8 : l1_of(logl), l2 = logl - l1;
       if (l1 > COLS_MAX_LOG || (l2 > COLS_MAX_LOG && !three)) {
@@ -781,11 +782,13 @@ struct Builder {
            outer * L2, inverse, L, L2 - 1, 0);
       // pass B: lines (o, k1), points t2 -> X[o][k1 + L1 k2]
       if (l2 > COLS_MAX_LOG) {
-        // the same as a strided axis: (outer, L2, inner L1) from Y to X,
-        // its own scratch above Y's
+        // the same as a strided axis: (outer, L2, inner L1) from Y to X, its
+        // own scratch above Y's; FP64 in place on Y, so that three passes take
+        // the scratch of two (16 x 2^20 at most 1.5% slower; FP32 16 x 2^21 260
+        // -> 266 us, not taken)
         const long long save = scr_base;
-        scr_base += 2 * outer * L;
-        axis(outer, L2, L1, S, B, inverse, L, b_bs);
+        if (!f64) scr_base += 2 * outer * L;
+        axis(outer, L2, L1, S, B, inverse, L, b_bs, f64);
         scr_base = save;
         return;
       }
@@ -807,10 +810,14 @@ struct Builder {
     }
     long long L1 = 1LL << l1, L2 = 1LL << l2;
     long long N = outer * L * inner;
-    View S = split_view(B_SCR, B_SCR, scr_base);
-    S.im.off = scr_base + N;
-    need_scratch(scr_base + 2 * N);
-    // pass A: lines (o, t2, m), points t1 (stride L2*inner) -> Y(k1, t2, m)
+    View S = A;
+    if (!over_a) {
+      S = split_view(B_SCR, B_SCR, scr_base);
+      S.im.off = scr_base + N;
+      need_scratch(scr_base + 2 * N);
+    }
+    // pass A: lines (o, t2, m), points t1 (stride L2*inner) -> Y(k1, t2, m),
+    // each line at its own addresses
     line(LK_C2C, true, false, l1, io(A, L2 * inner, 1, a_bs, l2 + lin, L2 * inner - 1),
          io(S, L2 * inner, 1, L * inner, l2 + lin, L2 * inner - 1), outer * L2 * inner, inverse, L,
          L2 - 1, lin);
