@@ -158,25 +158,19 @@ __device__ __forceinline__ double fx_to(fx a, int sc20) {
   return __hiloint2double(hi ? hi + sc20 : 0, __double2loint(d));
 }
 
-// The values seen, for their largest magnitude.  word(): its top bit is one
-// above that magnitude's, also in an OR of several.  MINMAX: the largest and
-// smallest high word, two three-way instructions per value; else an OR of x ^
-// 2x, four.  4096-point rows x 4096 239.0 -> 237.0 us with MINMAX, 512 x 32768
-// 165.7 -> 162.8, 2^20 r2c x 32 610 -> 600; the 256-point cols passes are
-// faster without (256^3 c2c 504 vs 508).
-template <bool MINMAX>
+// The values seen, for their largest magnitude: the largest and the smallest
+// high word, two three-way instructions per value (against an OR of x ^ 2x,
+// four: 4096-point rows x 4096 239.0 -> 237.0 us, 512 x 32768 165.7 -> 162.8,
+// 2^20 r2c x 32 610 -> 600, 256^3 502.5 -> 498.2).  word(): its top bit is one
+// above that magnitude's, also in an OR of several.
 struct FxMag {
   int hi = 0, lo = 0;
   __device__ __forceinline__ void add(fxc z) {
     const int a = fx_hi(z.x), b = fx_hi(z.y);
-    if constexpr (MINMAX) {
-      hi = __vimax3_s32(hi, a, b);
-      lo = __vimin3_s32(lo, a, b);
-    } else {
-      hi |= (a ^ (a + a)) | (b ^ (b + b));
-    }
+    hi = __vimax3_s32(hi, a, b);
+    lo = __vimin3_s32(lo, a, b);
   }
-  __device__ __forceinline__ int word() const { return MINMAX ? max(hi, ~lo) << 1 : hi; }
+  __device__ __forceinline__ int word() const { return max(hi, ~lo) << 1; }
 };
 
 // One value per line reduced over the line's threads.  Lines inside one warp
@@ -272,7 +266,7 @@ __device__ __forceinline__ void fx_stages(fxc (&v)[Sched64<LOGL>::E], int t, int
     constexpr int R = Sc::radix(S), NS = Sc::ns(S), E = Sc::E, T = Sc::T, B = E / R;
     constexpr bool LAST = S == Sc::NSTAGES - 1;
     using Ln = FxLine<T, C, COLS>;
-    FxMag<!(COLS && LOGL == 8)> seen;
+    FxMag seen;
 #pragma unroll
     for (int u = 0; u < B; u++) {
       const int b = t + T * u;
@@ -409,7 +403,7 @@ __device__ __forceinline__ void line_fx64_body(const LineParams& p, long long ct
     // same way (element L - i is this thread's alone in between).
     constexpr int IN = FX_TOP_C2R;
     sc += TOP - IN;
-    FxMag<!(COLS && LOGL == 8)> seen;
+    FxMag seen;
 #pragma unroll
     for (int e = 0; e < E; e++) v[e] = {fx_from<IN>(d[e].x, emax), fx_from<IN>(d[e].y, emax)};
 #pragma unroll
