@@ -1269,19 +1269,24 @@ int Plan::launch(const float* src_re, const float* src_im, float* dst_re, float*
       PairedTma pt;
       // (1024-point tiles take the pipelined kernel from two per CTA slot:
       // with one each it has nothing to prefetch and its float exchange
-      // costs more, 2048² c2r 0.0324 vs 0.0300 ms; the complex pass up to ten
-      // per slot, arrays that mostly stay in L2: 2^20 x 16 c2c 114 vs 119 us,
-      // but x 64 450 vs 419 and 1024² x 64 397 vs 365, where the CTAs' fixed
-      // shares of the tiles end unevenly)
+      // costs more, 2048² c2r 0.0324 vs 0.0300 ms.  The complex pass up to
+      // eight per slot: beyond, the arrays leave L2 and the CTAs' fixed shares
+      // of the tiles end unevenly.  Pipelined against one tile per CTA, us:
+      // 1024² x 5 (2.1 per slot) 27.4 vs 29.9, x 16 (6.7) 95.3 vs 96.5, x 20
+      // (8.4) 119.2 vs 117.7, x 24 (10.1) 143.4 vs 138.9, x 64 380 vs 346;
+      // 2^20 x 16 113.6 vs 117.1, x 20 141.0 vs 142.1, x 28 (11.8) 194.1 vs
+      // 191.4, x 64 449 vs 418; 1024 x 64 x 256 (6.7) 96.4 vs 97.8, x 384 (10)
+      // 143.5 vs 139.4.  The C2R pass at any number: 2048 x 1024 x 5 36.0 vs
+      // 38.3, x 32 180.9 vs 199.3)
       const long long slots = (long long)sm_count * op.k.pipe_ctas;
+      const bool pipe = op.k.pipe && sm_count > 0 &&
+                        (op.k.logl == 11 || (op.grid >= 2 * slots && (op.k.kind != LK_C2C || op.grid <= 8 * slots)));
+      const bool pipe_bulk_out = AFFT_PIPE_BULK_STORE && !op.k.tstore &&
+                                 ((op.k.kind == LK_C2C && (op.k.logl == 11 || AFFT_PIPE_BULK10)) ||
+                                  (op.k.kind == LK_C2R && op.k.logl == 10 && AFFT_PIPE_BULK_C2R10));
       if (op.k.paired_tma && tma_paired(p, op.k, &pt)) {
         launch_pass(op.k.paired_tma, op.grid, op.threads, op.k.paired_smem, st, p, pt);
-      } else if (op.k.pipe && sm_count > 0 && (op.k.logl == 11 || (op.grid >= 2 * slots && (op.k.kind != LK_C2C || op.grid <= 10 * slots))) &&
-          tma_tile(p, op.k, &tm) &&
-          (!(AFFT_PIPE_BULK_STORE && !op.k.tstore &&
-             ((op.k.kind == LK_C2C && (op.k.logl == 11 || AFFT_PIPE_BULK10)) ||
-              (op.k.kind == LK_C2R && op.k.logl == 10 && AFFT_PIPE_BULK_C2R10))) ||
-           tma_tile_out(p, op.k, &tmo))) {
+      } else if (pipe && tma_tile(p, op.k, &tm) && (!pipe_bulk_out || tma_tile_out(p, op.k, &tmo))) {
         // persistent: at most pipe_ctas CTAs per SM, each walking tiles gridDim.x apart
         const long long g = std::min<long long>(op.grid, slots);
         launch_pass(op.k.pipe, g, op.threads, op.k.pipe_smem, st, p, tm, tmo, op.grid);
