@@ -126,21 +126,25 @@ def supported(impl=afft_auto):
     return bool(lib().afft_supported(impl))
 
 
+_ndarray = None   # numpy.ndarray, from the first array on (numpy itself is not needed here)
+
+
 def ptr(a):
     """Address of a torch tensor, numpy array or int (None -> NULL)."""
+    global _ndarray
     if a is None:
         return None
     if isinstance(a, int):
         return a
-    f = getattr(a, "data_ptr", None)
-    if f is not None:
-        return f()
-    numpy = sys.modules.get("numpy")
-    if numpy is not None and type(a) is numpy.ndarray:
+    if type(a) is _ndarray:
         # a quarter of the time of a.ctypes.data; of arrays alone: others give
         # bytes here, or the address of a temporary (numpy's scalars)
         return a.__array_interface__["data"][0]
+    f = getattr(a, "data_ptr", None)
+    if f is not None:
+        return f()
     if hasattr(a, "ctypes"):
+        _ndarray = getattr(sys.modules.get("numpy"), "ndarray", None)
         return a.ctypes.data
     raise TypeError(type(a))
 
