@@ -354,21 +354,23 @@ __device__ __forceinline__ long long line_off(const LineIO& io, long long q) {
 __device__ __forceinline__ float2 ldg2(const float2* p) { return __ldg(p); }
 
 // Start of a kernel that a plan launches with programmatic stream
-// serialization: once every CTA of the previous launch has ended or is in its
-// last wave's drain, this grid's CTAs may take the free slots; they wait here
-// until that launch is complete and its results are visible.  The drain of
-// one pass then hides the launch and the start of the next: 256^3 c2c (three
-// passes) 133.6 -> 125.8 us a transform, 37 images of 512^2 68.9 -> 63.8,
-// 30011 real lines of 512 points 27.9 -> 25.3, 16384 lines of 4096 points
-// 174.2 -> 171.7, 128x128x256 x 2 real FP64 there and back 297 -> 281.  (No
-// explicit launch_dependents: it gains nothing over the trigger at each CTA's
-// end, and costs passes of many small CTAs 1.6 times their time, 2 x 1024
-// x 6895 c2c 154 -> 262.)
+// serialization.  No kernel triggers its dependants early, so this grid's CTAs
+// start once every CTA of the previous launch has ended; they wait here until
+// its results are visible.  What is hidden is the launch itself and the flush
+// at the end of the previous grid.  Without and with the attribute, us: 256^3
+// c2c (three passes) 130.8 -> 123.4, 37 images of 512^2 as pairs 59.2 -> 53.7,
+// 30011 real lines of 512 points 24.6 -> 21.6, 16384 lines of 4096 points 171.9
+// -> 169.1, 128x128x256 x 2 r2c FP64 133.3 -> 127.1, one 2^20 c2c 16.4 -> 12.3.
+// (An explicit launch_dependents at the start, which would let the next grid's
+// CTAs wait in the slots that this one's drain frees, gained nothing over this
+// and cost passes of many small CTAs 1.6 times their time, 2 x 1024 x 6895 c2c
+// 154 -> 262.)
 __device__ __forceinline__ void pdl_enter() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// Loads of the arrays a pass transforms.  Coherent ones: the previous launch
-// may still be writing them while this grid's CTAs start (pdl_enter), which
-// the read-only path does not allow for.  (Tables never change: __ldg.)
+// Loads of the arrays a pass transforms.  Coherent ones: the read-only path is
+// for data that do not change while the kernel runs, which begins before
+// pdl_enter's wait, and the compiler may move such a load above it.  (Tables
+// never change: __ldg.)
 __device__ __forceinline__ float ldin(const float* p) {
   float v;
   asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
@@ -400,14 +402,20 @@ namespace agb {
 //    2048-point R2C pass: 2^20 c2c x 16 127 -> 115, x 64 450 -> 420, 1024^2 x 64 368 -> 365, 512^2 x 37
 //    58.7 -> 57.0 (as pairs 63.5 -> 60.2), 2^20 r2c x 64 300 -> 286, c2r 334 ->
 //    297, 2048^2 c2r x 16 211 -> 192, r2c x 4 65.0 -> 62.2, 4096^2 r2c 74.4 ->
-//    72.8; not the paired real passes (2^20 r2c x 64 286 vs 318);
+//    72.8; not the paired real passes (2^20 r2c x 64 286 vs 318).  With LSU
+//    loads too (arrays that TMA does not take): 512^2 x 37 one float off 71.1 ->
+//    66.3, 1024^2 x 16 123.4 -> 115.8, as pairs 135.8 -> 118.0, r2c 56.2 ->
+//    52.4, c2r 59.4 -> 55.7, 2048 x 512 x 8 r2c 35.3 -> 31.4; only the four-step
+//    passes lose, 2^18 x 64 150.4 -> 152.1, as pairs 8 bytes off 120.1 -> 124.6;
 //  - complex rows of those lengths, whose lines then sit in a warp or half of
 //    one, without CTA barriers: 1024 x 65536 168 -> 153, as pairs 190 -> 154, 512 x 131072 157 ->
 //    154, as pairs 164 -> 154; and the 1024-point rows R2C pass, 2048 reals x
 //    65536 204 -> 170 (the 512-point one 186 -> 191, C2R level);
 //  - complex and R2C rows of 8192 and 16384 points (three stages against four):
 //    8192 x 8192 248 -> 210, as pairs 267 -> 224, 16384 x 4096 332 -> 306, 16384
-//    reals x 8192 304 -> 252; not the C2R rows (350 vs 361);
+//    reals x 8192 304 -> 252; not the C2R rows (350 vs 361); at few
+//    lines too, 8192 x 1 5.6 both ways, as pairs 6.0 -> 5.2, x 200 10.1 -> 8.3,
+//    16384 x 1 10.1 -> 9.2, 32768 reals x 1 11.5 -> 10.3;
 //  - of the queue's grouped kernels (GROUPED), which share the SMs with other
 //    groups, only the 1024-point rows (10000 mixed transforms 11.92 -> 11.73 ms,
 //    fewer level); the cols passes there are slower (1000 transforms 1005 vs

@@ -1222,9 +1222,9 @@ bool op_tables_ok(const Op& op) {
          (!op.k.plane_log1 || op.p.tw2);
 }
 
-// One launch of a plan.  Programmatic stream serialization: the kernel may
-// start while the launch before it drains (it waits for that one's results in
-// pdl_enter before touching any array).
+// One launch of a plan.  Programmatic stream serialization: the kernel's CTAs
+// may start as soon as those of the launch before it have ended (they wait for
+// its results in pdl_enter before touching any array).
 template <class... P>
 static void launch_pass(void (*fn)(P...), long long grid, int threads, size_t smem, cudaStream_t st,
                         const std::common_type_t<P>&... args) {
