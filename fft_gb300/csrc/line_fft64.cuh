@@ -16,7 +16,12 @@
 // Twiddles are computed in FP64 on the host and kept in 62-bit fixed point.
 // They travel in the LineParams / RealPassParams table fields (tw, tw_full,
 // rtw), which point to int4 arrays for these kernels; the four-step twiddle
-// always comes from the full matrix table tw_full[t2 * L + k].
+// always comes from the full matrix table tw_full[t2 * L + k].  The FP64 body
+// reads the stage and real twiddles as doubles, from double2 arrays in the
+// fields of the hi/lo pair, which FP64 plans do not have (tw_hi, tw_lo): two
+// conversions a twiddle on the FP64 pipe cost it 1.2 to 1.3 times its time
+// (real lines of 8 points x 2^21 218 us, with conversions 263; 4096-point lines
+// out of fixed point's range x 4096 1150 and 1477).
 #pragma once
 
 #include "line_fft.cuh"
@@ -73,6 +78,7 @@ __device__ __forceinline__ double2 zsub(double2 a, double2 b) { return make_doub
 __device__ __forceinline__ double2 zconj(double2 a) { return make_double2(a.x, -a.y); }
 __device__ __forceinline__ double2 zmul_negi(double2 a) { return make_double2(a.y, -a.x); }   // -i*a
 __device__ __forceinline__ double2 zswap(double2 a) { return make_double2(a.y, a.x); }
+__device__ __forceinline__ double2 ldz(const double2* p) { return __ldg(p); }
 // A root of unity from its fixed-point table entry (root_d in plan.cu): the
 // value is ((re high) * 2^32 + re low) / 2^62, likewise im.
 __device__ __forceinline__ double2 ldz(const int4* p) {
@@ -152,7 +158,7 @@ struct Smem64 {
 // slots u + B*r, applies W_{NS R}^{r (b mod NS)}, DFT-R, and scatters to
 // shared memory (non-last) or keeps the canonical layout (last).
 template <int R, int NS, int E, int T, bool LAST, class SM>
-__device__ __forceinline__ void stage64(double2 (&v)[E], int t, int c, const int4* tw, const SM& sm) {
+__device__ __forceinline__ void stage64(double2 (&v)[E], int t, int c, const double2* tw, const SM& sm) {
   constexpr int B = E / R;
 #pragma unroll
   for (int u = 0; u < B; u++) {
@@ -178,7 +184,7 @@ __device__ __forceinline__ void stage64(double2 (&v)[E], int t, int c, const int
 }
 
 template <int LOGL, bool WARP_ONLY, int S, class SM>
-__device__ __forceinline__ void run_stages64(double2 (&v)[Sched64<LOGL>::E], int t, int c, const int4* tw,
+__device__ __forceinline__ void run_stages64(double2 (&v)[Sched64<LOGL>::E], int t, int c, const double2* tw,
                                              const SM& sm) {
   using Sc = Sched64<LOGL>;
   if constexpr (S < Sc::NSTAGES) {
@@ -216,12 +222,12 @@ __device__ __forceinline__ void line_fft64_body(const LineParams& p, long long c
   constexpr bool WARP_ONLY = (!COLS && T <= 32) || (T * C <= 32);
   extern __shared__ __align__(1024) double2 smem64[];
   Smem64<L, C, COLS> sm{smem64};
-  const int4* tw = reinterpret_cast<const int4*>(p.tw);
-  const int4* rtw = reinterpret_cast<const int4*>(p.rtw);
+  const double2* tw = reinterpret_cast<const double2*>(p.tw_hi);
+  const double2* rtw = reinterpret_cast<const double2*>(p.tw_lo);
 
   const int tid = threadIdx.x;
   const int c = COLS ? (tid % C) : (tid / T);
-  const int t = COLS ? (tid / C) : (tid % T);
+  const int t = T == 1 ? 0 : COLS ? (tid / C) : (tid % T);   // (one thread per line: bins 0 and L known to the compiler)
   const long long q = cta * C + c;
   const bool active = q < p.nlines && (!only || only[c]);
 

@@ -337,7 +337,7 @@ __device__ __forceinline__ void line_fx64_body(const LineParams& p, long long ct
 
   const int tid = threadIdx.x;
   const int c = COLS ? (tid % C) : (tid / T);
-  const int t = COLS ? (tid / C) : (tid % T);
+  const int t = T == 1 ? 0 : COLS ? (tid / C) : (tid % T);   // (one thread per line: bins 0 and L known to the compiler)
   const long long q = cta * C + c;
   const bool active = q < p.nlines;
   const long long base = active ? line_off(p.in, q) : 0;
@@ -384,7 +384,14 @@ __device__ __forceinline__ void line_fx64_body(const LineParams& p, long long ct
   if constexpr (Ln::REG) top = Ln::in_regs_max(top);
   else Ln::publish_max(top, slots, c);
   const bool rare = __syncthreads_or(maybe);
-  if (rare && t == 0) odd_of[c] = fx_out_of_range(Ln::REG ? top : slots[c]);
+  if (rare) {
+    const bool odd = fx_out_of_range(Ln::REG ? top : slots[c]);
+    if (__syncthreads_and(odd || !active)) {   // no line is left to the fixed-point form
+      line_fft64_general<LOGL, C, COLS, KIND, TSTORE>(p, cta, nullptr);
+      return;
+    }
+    if (t == 0) odd_of[c] = odd;
+  }
   if constexpr (!Ln::REG) top = slots[c];
   constexpr int TOP = fx_top<LOGL>();
   const int emax = max(top >> 20, FX_EXP_MIN);   // (a line of zeros: every element shifts out)

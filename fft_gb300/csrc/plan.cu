@@ -83,7 +83,7 @@ static float2 root_f(long long m, long long N) {
 
 struct TableCache {
   std::mutex mu;
-  std::map<std::pair<int, long long>, void*> tables;  // (device * 8 + type, key)
+  std::map<std::pair<int, long long>, void*> tables;  // (device * 16 + type, key)
 };
 static TableCache& tcache() {
   static TableCache* c = new TableCache();  // never destroyed: outlives static plans
@@ -91,7 +91,7 @@ static TableCache& tcache() {
 }
 
 // Device copy of table (type, key) on the current device; `make` builds the
-// host table (a std::vector of float2 or int4) on the first request only.
+// host table (a std::vector of float2, int4 or double2) on the first request only.
 template <class F>
 static auto cached_table(int type, long long key, F make) -> const typename decltype(make())::value_type* {
   using V = typename decltype(make())::value_type;
@@ -99,7 +99,7 @@ static auto cached_table(int type, long long key, F make) -> const typename decl
   cudaGetDevice(&dev);
   auto& C = tcache();
   std::lock_guard<std::mutex> g(C.mu);
-  auto id = std::make_pair(dev * 8 + type, key);
+  auto id = std::make_pair(dev * 16 + type, key);
   auto it = C.tables.find(id);
   if (it != C.tables.end()) return static_cast<const V*>(it->second);
   const std::vector<V> host = make();
@@ -301,6 +301,11 @@ static void split62(double v, bool away, int* hi, int* lo) {
   // products' exact quarters round their ties by the sign of the data
   if (*lo == 0 && *hi != 0) *lo = (*hi > 0) == away ? 1 : -1;
 }
+static double2 root_z(long long m, long long N) {
+  double c, s;
+  unit_root(m, N, &c, &s);
+  return make_double2(c, s);
+}
 static int4 root_d(long long m, long long N, bool away = false) {
   double c, s;
   unit_root(m, N, &c, &s);
@@ -310,34 +315,45 @@ static int4 root_d(long long m, long long N, bool away = false) {
   return w;
 }
 
-template <int LOGL>
-static std::vector<int4> stage_table64() {
+template <int LOGL, class V, class Root>
+static std::vector<V> stage_table64(Root root) {
   using S = Sched64<LOGL>;
-  std::vector<int4> t(S::twsize());
+  std::vector<V> t(S::twsize());
   for (int s = 0; s < S::NSTAGES; s++) {
     int ns = S::ns(s), R = S::radix(s);
     if (ns == 1) continue;
     int off = S::twoff(s);
     for (int r = 1; r < R; r++)
       for (int k = 0; k < ns; k++)   // (away from zero for r = 1, 2, 5: fx_sar in line_fx64.cuh)
-        t[off + (r - 1) * ns + k] = root_d((long long)r * k, (long long)ns * R, (0x26 >> r) & 1);
+        t[off + (r - 1) * ns + k] = root((long long)r * k, (long long)ns * R, (0x26 >> r) & 1);
   }
   return t;
 }
 
-template <int... Ls>
-static std::vector<int4> stage_table64_dispatch(int logl, std::integer_sequence<int, Ls...>) {
-  std::vector<int4> out;
-  ((logl == Ls ? (void)(out = stage_table64<Ls>()) : (void)0), ...);
+template <class V, class Root, int... Ls>
+static std::vector<V> stage_table64_of(int logl, Root root, std::integer_sequence<int, Ls...>) {
+  std::vector<V> out;
+  ((logl == Ls ? (void)(out = stage_table64<Ls, V>(root)) : (void)0), ...);
   return out;
 }
-
-std::vector<int4> stage_table64_host(int logl) {
-  return stage_table64_dispatch(logl, std::make_integer_sequence<int, ROWS_MAX_LOG64 + 1>{});
-}
+using Lines64 = std::make_integer_sequence<int, ROWS_MAX_LOG64 + 1>;
 
 const int4* stage_twiddles64(int logl) {
-  return cached_table(5, logl, [&] { return stage_table64_host(logl); });
+  return cached_table(5, logl, [&] { return stage_table64_of<int4>(logl, root_d, Lines64{}); });
+}
+
+const double2* stage_twiddles64_d(int logl) {
+  return cached_table(8, logl, [&] {
+    return stage_table64_of<double2>(logl, [](long long m, long long N, bool) { return root_z(m, N); }, Lines64{});
+  });
+}
+
+const double2* real_twiddles64_d(long long L) {
+  return cached_table(9, L, [&] {
+    std::vector<double2> t(L);
+    for (long long k = 0; k < L; k++) t[k] = root_z(k, 2 * L);
+    return t;
+  });
 }
 
 const int4* real_twiddles64(long long L) {
@@ -602,8 +618,10 @@ struct Builder {
         P.has_tma = true;
       }
       if (f64) {
-        // the FP64 kernels read int4 tables through the same fields
+        // the FP64 kernels read int4 and double2 tables through the same fields
         op.p.tw = reinterpret_cast<const float2*>(stage_twiddles64(op.k.stage_logl));
+        op.p.tw_hi = reinterpret_cast<const float2*>(stage_twiddles64_d(op.k.stage_logl));
+        if (real_L) op.p.tw_lo = reinterpret_cast<const float2*>(real_twiddles64_d(real_L));
         if (tw_n) op.p.tw_full = reinterpret_cast<const float2*>(fourstep_full_table64(tw_n, tw_qmask + 1));
         if (real_L) op.p.rtw = reinterpret_cast<const float2*>(real_twiddles64(real_L));
       } else {
@@ -626,7 +644,7 @@ struct Builder {
     op.grid = (nlines + op.k.lines_per_cta - 1) / op.k.lines_per_cta * op.k.halves;
     op.threads = op.k.threads;
     op.smem = op.k.smem;
-    if (!dry && (!op.p.tw || (tw_n && !f64 && (!op.p.tw_hi || !op.p.tw_lo)) ||
+    if (!dry && (!op.p.tw || (f64 ? !op.p.tw_hi || (real_L && !op.p.tw_lo) : tw_n && (!op.p.tw_hi || !op.p.tw_lo)) ||
                  (tw_n && (f64 || tw_n <= kFullTableMax) && !op.p.tw_full) || (real_L && !op.p.rtw))) {
       fail("twiddle table allocation failed");
       return;

@@ -166,7 +166,9 @@ const float2* fourstep_full_table(long long N, long long L2);
 const int4* stage_twiddles64(int logl);
 const int4* real_twiddles64(long long L);
 const int4* fourstep_full_table64(long long N, long long L2);
-std::vector<int4> stage_table64_host(int logl);
+// the first two as doubles, for the FP64 body of the line kernels
+const double2* stage_twiddles64_d(int logl);
+const double2* real_twiddles64_d(long long L);
 std::vector<float2> fourstep_full_table_host(long long N, long long L2);
 // The same tables on the host, without touching the device.
 std::vector<float2> stage_table_host(int logl);
